@@ -394,45 +394,16 @@ __global__ void heavy_runs_kernel(const int64_t* __restrict__ k, int64_t n, int6
     }
 }
 
-__global__ void to_signed_kernel(const uint64_t* __restrict__ in, int64_t n, int64_t* __restrict__ out)
-{
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        out[i] = from_sortable(in[i]);
-}
-
-__global__ void to_sortable_kernel(const int64_t* __restrict__ in, int64_t n, uint64_t* __restrict__ out)
-{
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        out[i] = to_sortable(in[i]);
-}
-
 // Sorted copy of n device keys into *sorted (device, caller frees).
 int sort_keys(pyg_ctx* ctx, const int64_t* keys, int64_t n, int64_t** sorted)
 {
-    uint64_t* buf;
-    int rc = dalloc(ctx, (void**)&buf, (size_t)2 * (n > 0 ? n : 1) * 8);
+    int rc = dalloc(ctx, (void**)sorted, (size_t)(n > 0 ? n : 1) * 8);
     if (rc) return rc;
-    int g = grid_for(ctx, n, 256, 4, 8);
-    if (n > 0) {
-        to_sortable_kernel<<<g, 256, 0, ctx->stream>>>(keys, n, buf);
-        PYG_LAUNCHED(ctx);
+    if ((rc = radix_sort8_to(ctx, (const uint64_t*)keys, (uint64_t*)*sorted, n, true))) {
+        dfree(ctx, *sorted);
+        *sorted = nullptr;
     }
-    int b = 0, e = 0, alt = 0;
-    if (!(rc = key_bit_range(ctx, buf, n, &b, &e))) rc = radix_sort_pairs(ctx, buf, nullptr, buf + n, nullptr, n, b, e, &alt);
-    if (rc) {
-        dfree(ctx, buf);
-        return rc;
-    }
-    if ((rc = dalloc(ctx, (void**)sorted, (size_t)(n > 0 ? n : 1) * 8))) {
-        dfree(ctx, buf);
-        return rc;
-    }
-    if (n > 0) {
-        to_signed_kernel<<<g, 256, 0, ctx->stream>>>(alt ? buf + n : buf, n, *sorted);
-        PYG_LAUNCHED(ctx);
-    }
-    dfree(ctx, buf);
-    return PYG_OK;
+    return rc;
 }
 
 // Device workspace for one forward/backward pass over a sorted sample.
@@ -579,6 +550,7 @@ int pyg_cdf_train(pyg_ctx* ctx, const int64_t* sample_keys, int64_t n, const pyg
         PYG_CUDA(cudaMemcpyAsync(hruns, runs, (size_t)cap * 24, cudaMemcpyDeviceToHost, ctx->stream));
         PYG_CUDA(cudaStreamSynchronize(ctx->stream));
         dfree(ctx, runs);
+        if ((rc = sort_status(ctx))) break;
         m->kmin = hends[0];
         m->kmax = hends[1];
         m->distinct = (int64_t)hst[0];
@@ -1261,7 +1233,7 @@ int pyg_sampled_splitters(pyg_ctx* ctx, const int64_t* sample_keys, int64_t n, i
     PYG_CUDA(cudaStreamSynchronize(ctx->stream));
     dfree(ctx, d);
     dfree(ctx, sorted);
-    return PYG_OK;
+    return sort_status(ctx);
 }
 
 int pyg_cdf_estimate_distinct(pyg_ctx* ctx, const pyg_cdf* m, int64_t population, int64_t* out)

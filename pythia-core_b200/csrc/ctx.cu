@@ -195,7 +195,11 @@ int pyg_ctx_create(int device, pyg_ctx** out)
     c->stream = c->own_stream;
     c->pinned_bytes = kPinnedScalarBytes + kPinnedStageBytes + kPinnedUploadBytes;
     e = cudaMallocHost(&c->pinned, c->pinned_bytes);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&c->dcounters, 4096);
+    if (e == cudaSuccess) {
+        memset(c->pinned, 0, kPinnedScalarBytes);
+        e = cudaMalloc((void**)&c->dcounters, 4096);
+    }
+    if (e == cudaSuccess) e = cudaMemset(c->dcounters, 0, 4096);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking);
     for (int i = 0; i < 2 && e == cudaSuccess; ++i) {
         e = cudaEventCreateWithFlags(&c->copied[i], cudaEventDisableTiming);

@@ -183,7 +183,7 @@ __device__ __forceinline__ void write_group(uint8_t* dst, const OutSpec& o, uint
 // Compaction: occupied slots -> output rows (unordered), or -> (sortable
 // key, slot) pairs for the ordered path.
 __global__ void gb_compact_kernel(const ulonglong4* __restrict__ table, uint64_t cap, OutSpec o, uint8_t* out,
-                                  int64_t out_cap, uint64_t* skeys, uint64_t* sidx, unsigned long long* cursor)
+                                  int64_t out_cap, ulonglong2* items, unsigned long long* cursor)
 {
     const unsigned lane = threadIdx.x & 31;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
@@ -198,20 +198,19 @@ __global__ void gb_compact_kernel(const ulonglong4* __restrict__ table, uint64_t
         base = __shfl_sync(0xffffffffu, base, 0);
         if (!occ) continue;
         int64_t p = (int64_t)(base + __popc(m & ((1u << lane) - 1)));
-        if (skeys) {
-            skeys[p] = packed_to_sortable(e.x, o.nkeys);
-            sidx[p] = s;
+        if (items) {
+            items[p] = make_ulonglong2(packed_to_sortable(e.x, o.nkeys), s);
         } else if (p < out_cap) {
             write_group(out + p * o.tb, o, e.x, e.y, e.z);
         }
     }
 }
 
-__global__ void gb_write_sorted_kernel(const ulonglong4* __restrict__ table, const uint64_t* __restrict__ sidx,
+__global__ void gb_write_sorted_kernel(const ulonglong4* __restrict__ table, const ulonglong2* __restrict__ items,
                                        int64_t n, int64_t sentinel_pos, OutSpec o, uint64_t sent_key,
                                        uint64_t sent_sum, uint64_t sent_cnt, uint8_t* out)
 {
-    // Rows before sentinel_pos come from sidx[i], the sentinel group (if any)
+    // Rows before sentinel_pos come from slot items[i].y, the sentinel group (if any)
     // sits at sentinel_pos, the rest shift by one.
     int64_t total = n + (sentinel_pos >= 0 ? 1 : 0);
     for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < total; r += (int64_t)gridDim.x * blockDim.x) {
@@ -220,17 +219,17 @@ __global__ void gb_write_sorted_kernel(const ulonglong4* __restrict__ table, con
             continue;
         }
         int64_t i = (sentinel_pos >= 0 && r > sentinel_pos) ? r - 1 : r;
-        ulonglong4 e = table[sidx[i]];
+        ulonglong4 e = table[items[i].y];
         write_group(out + r * o.tb, o, e.x, e.y, e.z);
     }
 }
 
-__global__ void count_below_kernel(const uint64_t* __restrict__ skeys, int64_t n, uint64_t pivot,
+__global__ void count_below_kernel(const ulonglong2* __restrict__ items, int64_t n, uint64_t pivot,
                                    unsigned long long* out)
 {
     unsigned long long c = 0;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        c += skeys[i] < pivot;
+        c += items[i].x < pivot;
     c = warp_sum_u64(c);
     if ((threadIdx.x & 31) == 0 && c) atomicAdd(out, c);
 }
@@ -397,7 +396,7 @@ extern "C" int pyg_groupby(pyg_ctx* ctx, const pyg_rel* in, const int32_t* key_c
     int cgrid = grid_for(ctx, (int64_t)cap, threads, 4, 8);
     if (!sort_by_key) {
         gb_compact_kernel<<<cgrid, threads, 0, ctx->stream>>>(table, cap, o, (uint8_t*)out, out_capacity, nullptr,
-                                                              nullptr, cursor);
+                                                              cursor);
         PYG_LAUNCHED(ctx);
         if (sent_cnt) {
             uint8_t row[24];
@@ -414,19 +413,16 @@ extern "C" int pyg_groupby(pyg_ctx* ctx, const pyg_rel* in, const int32_t* key_c
             PYG_CUDA(cudaMemcpyAsync(dst, h + 16, oo.tb, cudaMemcpyHostToDevice, ctx->stream));
         }
     } else {
-        uint64_t* buf = nullptr;
+        ulonglong2 *buf = nullptr, *sorted = nullptr;
         int64_t g = (int64_t)groups;
-        if ((rc = dalloc(ctx, (void**)&buf, (size_t)4 * (g > 0 ? g : 1) * sizeof(uint64_t)))) {
+        if ((rc = dalloc(ctx, (void**)&buf, (size_t)2 * (g > 0 ? g : 1) * sizeof(ulonglong2)))) {
             dfree(ctx, table);
             R.release(ctx);
             return rc;
         }
-        uint64_t *k0 = buf, *v0 = buf + g, *k1 = buf + 2 * g, *v1 = buf + 3 * g;
-        gb_compact_kernel<<<cgrid, threads, 0, ctx->stream>>>(table, cap, o, nullptr, 0, k0, v0, cursor);
+        gb_compact_kernel<<<cgrid, threads, 0, ctx->stream>>>(table, cap, o, nullptr, 0, buf, cursor);
         PYG_LAUNCHED(ctx);
-        int b = 0, e = 0, alt = 0;
-        rc = key_bit_range(ctx, k0, g, &b, &e);
-        if (!rc) rc = radix_sort_pairs(ctx, k0, v0, k1, v1, g, b, e, &alt);
+        rc = radix_sort16_swap(ctx, buf, buf + g, g, 0, &sorted);
         int64_t sentinel_pos = -1;
         if (!rc && sent_cnt) {
             // Place the sentinel group: number of sorted keys below it.
@@ -434,7 +430,7 @@ extern "C" int pyg_groupby(pyg_ctx* ctx, const pyg_rel* in, const int32_t* key_c
             unsigned long long* c = ctx->dcounters + 56;
             cudaMemsetAsync(c, 0, 8, ctx->stream);
             count_below_kernel<<<grid_for(ctx, g > 0 ? g : 1, threads, 4, 8), threads, 0, ctx->stream>>>(
-                alt ? k1 : k0, g, pivot, c);
+                sorted, g, pivot, c);
             PYG_LAUNCHED(ctx);
             cudaMemcpyAsync(h + 8, c, 8, cudaMemcpyDeviceToHost, ctx->stream);
             cudaStreamSynchronize(ctx->stream);
@@ -442,7 +438,7 @@ extern "C" int pyg_groupby(pyg_ctx* ctx, const pyg_rel* in, const int32_t* key_c
         }
         if (!rc && total > 0) {
             gb_write_sorted_kernel<<<grid_for(ctx, total, threads, 4, 8), threads, 0, ctx->stream>>>(
-                table, alt ? v1 : v0, g, sentinel_pos, o, kEmptyKey, sent_sum, sent_cnt, (uint8_t*)out);
+                table, sorted, g, sentinel_pos, o, kEmptyKey, sent_sum, sent_cnt, (uint8_t*)out);
             PYG_LAUNCHED(ctx);
         }
         dfree(ctx, buf);
@@ -450,5 +446,5 @@ extern "C" int pyg_groupby(pyg_ctx* ctx, const pyg_rel* in, const int32_t* key_c
     dfree(ctx, table);
     R.release(ctx);
     PYG_CUDA(cudaStreamSynchronize(ctx->stream));
-    return rc;
+    return rc ? rc : sort_status(ctx);
 }

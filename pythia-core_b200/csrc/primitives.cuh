@@ -10,15 +10,19 @@ namespace pyg {
 int exclusive_scan_u64(pyg_ctx* ctx, const unsigned long long* in, unsigned long long* out, int64_t n,
                        unsigned long long* total_dev);
 
-// Stable LSD radix sort of (key, value) pairs by unsigned key over bits
-// [begin_bit, end_bit).  Sorted data ends in (keys, vals) or (keys_alt,
-// vals_alt); *in_alt tells which.  vals may be null (keys only).
-int radix_sort_pairs(pyg_ctx* ctx, uint64_t* keys, uint64_t* vals, uint64_t* keys_alt, uint64_t* vals_alt,
-                     int64_t n, int begin_bit, int end_bit, int* in_alt);
-
-// [begin, end) bit range over which the n keys differ (computed on device,
-// read back with a stream sync).  begin == end when all keys are equal.
-int key_bit_range(pyg_ctx* ctx, const uint64_t* keys, int64_t n, int* begin_bit, int* end_bit);
+// Stable LSD radix sorts (sort.cu) of 16-byte elements by 64-bit word
+// `field` (0 or 1), and of bare 64-bit keys.  Each reads the key range back
+// (one stream synchronisation) beyond 4096 elements.  After the caller's
+// next synchronisation of the stream, sort_status reports a pass whose
+// bounded device-side wait gave up.
+//
+// Into out (may not alias in).
+int radix_sort16_to(pyg_ctx* ctx, const ulonglong2* in, ulonglong2* out, int64_t n, int field, bool is_signed);
+int radix_sort8_to(pyg_ctx* ctx, const uint64_t* in, uint64_t* out, int64_t n, bool is_signed);
+// Unsigned order, both buffers overwritten; *result is the one holding the
+// sorted elements.
+int radix_sort16_swap(pyg_ctx* ctx, ulonglong2* a, ulonglong2* b, int64_t n, int field, ulonglong2** result);
+int sort_status(pyg_ctx* ctx);
 
 // Order-preserving map of a signed 64-bit value to an unsigned one.
 __host__ __device__ __forceinline__ uint64_t to_sortable(int64_t v)
@@ -47,7 +51,7 @@ constexpr int64_t CDF_MPSM_SAMPLE = (int64_t)1 << 21;
 int estimate_distinct_keys(pyg_ctx* ctx, const uint8_t* base, int64_t n, int32_t tb, const KeySpec& ks,
                            int64_t* out);
 
-// Gather rows: out[i] = in[idx[i]] for tuples of tb bytes.
-int gather_rows(pyg_ctx* ctx, const uint8_t* in, const uint64_t* idx, int64_t n, int32_t tb, uint8_t* out);
+// Gather rows: out[i] = in[items[i].y] for tuples of tb bytes.
+int gather_rows(pyg_ctx* ctx, const uint8_t* in, const ulonglong2* items, int64_t n, int32_t tb, uint8_t* out);
 
 }  // namespace pyg

@@ -47,7 +47,7 @@ __global__ void __launch_bounds__(TK_THREADS) tk_hist_kernel(const uint8_t* __re
 // Appends (order key, row) of every tuple whose top bits are <= bstar.
 __global__ void __launch_bounds__(TK_THREADS) tk_select_kernel(const uint8_t* __restrict__ base, int64_t n, int32_t tb,
                                                                KeySpec ks, int asc, unsigned bstar,
-                                                               uint64_t* __restrict__ okey, uint64_t* __restrict__ row,
+                                                               ulonglong2* __restrict__ items,
                                                                unsigned long long* __restrict__ cursor)
 {
     const unsigned lane = threadIdx.x & 31;
@@ -67,21 +67,17 @@ __global__ void __launch_bounds__(TK_THREADS) tk_select_kernel(const uint8_t* __
         if (lane == 0) at = atomicAdd(cursor, (unsigned long long)__popc(m));
         at = __shfl_sync(0xffffffffu, at, 0);
         if (take) {
-            const unsigned long long p = at + __popc(m & ((1u << lane) - 1u));
-            okey[p] = k;
-            row[p] = (uint64_t)i;
+            items[at + __popc(m & ((1u << lane) - 1u))] = make_ulonglong2(k, (uint64_t)i);
         }
     }
 }
 
 // Every tuple's (order key, row), for limit >= n.
 __global__ void tk_all_kernel(const uint8_t* __restrict__ base, int64_t n, int32_t tb, KeySpec ks, int asc,
-                              uint64_t* __restrict__ okey, uint64_t* __restrict__ row)
+                              ulonglong2* __restrict__ items)
 {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        okey[i] = tk_order(base + i * tb, ks, asc);
-        row[i] = (uint64_t)i;
-    }
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        items[i] = make_ulonglong2(tk_order(base + i * tb, ks, asc), (uint64_t)i);
 }
 
 }  // namespace pyg
@@ -112,7 +108,7 @@ extern "C" int pyg_sortlimit(pyg_ctx* ctx, const pyg_rel* in, const int32_t* key
     if ((rc = R.stage(ctx, in))) return rc;
     const uint8_t* base = (const uint8_t*)R.rel.base;
     const int32_t tb = in->tuple_bytes;
-    uint64_t* pairs = nullptr;  // okey, row, okey_alt, row_alt
+    ulonglong2* pairs = nullptr;  // (order key, row) items, then as many again to sort into
     unsigned long long* hist = nullptr;
     int64_t w = n;              // pairs selected
     do {
@@ -133,33 +129,26 @@ extern "C" int pyg_sortlimit(pyg_ctx* ctx, const pyg_rel* in, const int32_t* key
             unsigned long long* cursor = ctx->dcounters + 120;
             PYG_CUDA(cudaMemsetAsync(cursor, 0, 8, ctx->stream));
             tk_select_kernel<<<grid_for(ctx, n, TK_THREADS, 8, 4), TK_THREADS, 0, ctx->stream>>>(
-                base, n, tb, ks, asc, bstar, pairs, pairs + w, cursor);
+                base, n, tb, ks, asc, bstar, pairs, cursor);
             PYG_LAUNCHED(ctx);
         } else {
             if ((rc = dalloc(ctx, (void**)&pairs, (size_t)n * 32))) break;
-            tk_all_kernel<<<grid_for(ctx, n, 256, 4, 8), 256, 0, ctx->stream>>>(base, n, tb, ks, asc, pairs,
-                                                                                pairs + n);
+            tk_all_kernel<<<grid_for(ctx, n, 256, 4, 8), 256, 0, ctx->stream>>>(base, n, tb, ks, asc, pairs);
             PYG_LAUNCHED(ctx);
         }
         // Sort by row, then (stably) by order key: (order key, row) order.
-        uint64_t *key = pairs, *row = pairs + w, *key2 = pairs + 2 * w, *row2 = pairs + 3 * w;
-        int rbits = 1;
-        while (rbits < 64 && ((uint64_t)1 << rbits) < (uint64_t)n) ++rbits;
-        int alt = 0;
-        if ((rc = radix_sort_pairs(ctx, row, key, row2, key2, w, 0, rbits, &alt))) break;
-        if (alt) {
-            std::swap(row, row2);
-            std::swap(key, key2);
+        ulonglong2 *sorted = pairs;
+        if (k < n) {  // the selection appended them in any order
+            if ((rc = radix_sort16_swap(ctx, pairs, pairs + w, w, 1, &sorted))) break;
         }
-        int b0 = 0, b1 = 0;
-        if ((rc = key_bit_range(ctx, key, w, &b0, &b1))) break;
-        if ((rc = radix_sort_pairs(ctx, key, row, key2, row2, w, b0, b1, &alt))) break;
-        if (alt) row = row2;
-        rc = gather_rows(ctx, base, row, k, tb, (uint8_t*)out);
+        ulonglong2* other = sorted == pairs ? pairs + w : pairs;
+        if ((rc = radix_sort16_swap(ctx, sorted, other, w, 0, &sorted))) break;
+        rc = gather_rows(ctx, base, sorted, k, tb, (uint8_t*)out);
     } while (0);
     dfree(ctx, hist);
     dfree(ctx, pairs);
     R.release(ctx);
-    if (!rc) PYG_CUDA(cudaStreamSynchronize(ctx->stream));
-    return rc;
+    if (rc) return rc;
+    PYG_CUDA(cudaStreamSynchronize(ctx->stream));
+    return sort_status(ctx);
 }
