@@ -437,16 +437,16 @@ int groupby16_fill(pyg_ctx* ctx, const void* in, int64_t n, int want_sum, int64_
         PYG_CUDA(cudaMemcpyAsync(h.data(), hist, (size_t)F * 8, cudaMemcpyDeviceToHost, ctx->stream));
         PYG_CUDA(cudaStreamSynchronize(ctx->stream));
         RJLayout L;
-        if (sample) layout_sampled(h, step, C, sub, L);
-        else layout_exact(h, C, sub, L);
+        if (sample) layout_sampled(h, step, n, C, sub, L);
+        else layout_exact(h, n, C, sub, L);
         unsigned* hp = (unsigned*)ctx->pinned + 64;
         for (int attempt = 0; attempt < 2; ++attempt) {
             if ((rc = upload_layout(ctx, L, d, F, C, n))) break;
             dfree(ctx, P1);
             dfree(ctx, P2);
             P1 = P2 = nullptr;
-            if ((rc = dalloc(ctx, &P1, (size_t)L.p1 * 16))) break;
-            if (two && (rc = dalloc(ctx, &P2, (size_t)L.p2 * 16))) break;
+            if ((rc = dalloc(ctx, &P1, pass_bytes(L, L.p1)))) break;
+            if (two && (rc = dalloc(ctx, &P2, pass_bytes(L, L.p2)))) break;
             if ((rc = run_passes(ctx, src, n, L, d, two, FB, CB, P1, P2, pflags, pflags + 1))) break;
             PYG_CUDA(cudaMemcpyAsync(hp, pflags, 8, cudaMemcpyDeviceToHost, ctx->stream));
             if (L.sampled) {
@@ -464,7 +464,7 @@ int groupby16_fill(pyg_ctx* ctx, const void* in, int64_t n, int want_sum, int64_
             if ((rc = hist_launch(ctx, src, n, 1, FB, hist))) break;
             PYG_CUDA(cudaMemcpyAsync(h.data(), hist, (size_t)F * 8, cudaMemcpyDeviceToHost, ctx->stream));
             PYG_CUDA(cudaStreamSynchronize(ctx->stream));
-            layout_exact(h, C, sub, L);
+            layout_exact(h, n, C, sub, L);
             PYG_CUDA(cudaMemsetAsync(pflags, 0, 8, ctx->stream));
         }
         if (rc) break;

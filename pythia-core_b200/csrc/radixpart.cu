@@ -15,15 +15,7 @@
 
 namespace pyg {
 
-#ifndef PYG_RJ_PT_MINB
-#define PYG_RJ_PT_MINB 2
-#endif
-#ifndef PYG_RJ_STAGES
-#define PYG_RJ_STAGES 2
-#endif
-constexpr int RJ_STAGES = PYG_RJ_STAGES;                               // input tiles in flight per partition CTA
 constexpr unsigned long long kBulkWaitNs = 2000000000ULL;  // 2 s
-constexpr unsigned long long kSkipRun = 1ULL << 63;          // gdelta of a run that is not written
 
 __device__ __forceinline__ unsigned rj_bin(uint64_t h, int shift, unsigned mask)
 {
@@ -123,14 +115,16 @@ __global__ void rj_hist_sum_kernel(const unsigned* __restrict__ part, int nrow, 
 // at most 2^8 segments): tiles[C] is the pass's tile count.  Counts are
 // first clamped to their region's capacity, so a region that overflowed
 // (its result is discarded and redone) is never read past its end.
-__global__ void rj_tile_prefix_kernel(unsigned long long* __restrict__ count, const unsigned long long* __restrict__ cap,
+__global__ void rj_tile_prefix_kernel(const unsigned long long* __restrict__ cursor, int cstride,
+                                      unsigned long long* __restrict__ count, const unsigned long long* __restrict__ cap,
                                       int C, int tile, unsigned long long* __restrict__ tiles)
 {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     unsigned long long t = 0;
     tiles[0] = 0;
     for (int c = 0; c < C; ++c) {
-        const unsigned long long n = count[c] < cap[c] ? count[c] : cap[c];
+        const unsigned long long reached = cursor[(size_t)c * cstride];
+        const unsigned long long n = reached < cap[c] ? reached : cap[c];
         count[c] = n;
         t += (n + tile - 1) / tile;
         tiles[c + 1] = t;
@@ -149,16 +143,19 @@ struct RJPass {
     const unsigned long long* seg_start;  // nseg + 1 exact segment bounds in `in`
     const unsigned long long* seg_tile0;  // nseg + 1 prefix of tiles per segment
     int nseg;
+    int tile;                             // elements per tile (at most the kernel's largest)
     int shift;
     unsigned mask;
     int lbits;
     const unsigned long long* bin_start;  // output region start per output bin
-    unsigned long long* cursor;           // per output bin, zeroed before the pass
+    unsigned long long* cursor;           // per output bin, zeroed before the pass; bin b at b * cstride
+    int cstride;
     unsigned* err;                        // set if a tile's bulk copy never completed
     // Optional (null when offsets are exact):
     const unsigned long long* seg_count;  // tuples in each segment (segment end = start + count)
     const unsigned long long* bin_cap;    // region capacity per output bin
-    unsigned* ovf;                        // set when a bin outgrows its region (the run is not written)
+    unsigned* ovf;                        // set when a bin outgrows its region
+    unsigned long long dump;              // first of RJ_DUMP elements of `out` that take the runs of such bins
     const unsigned long long* ntiles_dev; // tile count read on the device
     // Range mode (nsplit > 0): bin = number of splitters <= key among the
     // segment's nsplit splitters, split + seg * 2^lbits (one segment: split).
@@ -177,12 +174,17 @@ struct RJPass {
 // intermediates) or packed 8-byte words, and writes either.  Packed input
 // tiles hold 4096 words (bins of at most 2^8, so the staged bin index is
 // one byte); 16-byte tiles hold 2048 tuples.  Both fit two CTAs per SM.
-template <bool IN8, bool OUT8>
+// How a pass computes a tuple's bin, fixed per kernel instance so that no
+// per-tuple branch chooses it.
+enum RJMode { RJ_MODE_HASH = 0, RJ_MODE_MODEL = 1, RJ_MODE_RANGE = 2 };
+
+template <bool IN8, bool OUT8, int MODE>
 struct RJFmt {
     using In = typename std::conditional<IN8, unsigned long long, longlong2>::type;
     using Out = typename std::conditional<OUT8, unsigned long long, longlong2>::type;
     using Bin = typename std::conditional<IN8, unsigned char, unsigned short>::type;
-    static constexpr int TILE = IN8 ? RJ_TILE8 : RJ_TILE;
+    static constexpr int TILE =
+        IN8 ? (MODE == RJ_MODE_HASH ? RJ_TILE_8 : RJ_TILE_8M) : (!OUT8 ? RJ_TILE_U : (MODE == RJ_MODE_HASH ? RJ_TILE_P : RJ_TILE_PM));  // the largest
 };
 
 __device__ __forceinline__ long long rj_key(const longlong2& t, unsigned long long) { return t.x; }
@@ -208,7 +210,6 @@ struct RJSegCursor {
     long long start, end;  // the segment's elements in `in`
 };
 
-template <int TILE>
 __device__ RJTileRange rj_tile_range(const RJPass& a, RJSegCursor& c, long long tile)
 {
     if (tile >= c.t1) {
@@ -223,34 +224,65 @@ __device__ RJTileRange rj_tile_range(const RJPass& a, RJSegCursor& c, long long 
     }
     RJTileRange r;
     r.seg = c.seg;
-    r.begin = c.start + (tile - c.t0) * TILE;
-    r.end = min(r.begin + TILE, c.end);
+    r.begin = c.start + (tile - c.t0) * a.tile;
+    r.end = min(r.begin + a.tile, c.end);
     return r;
 }
 
-// Shared memory of one partition CTA: a ring of RJ_STAGES input tiles that
-// bulk copies fill ahead of use, the grouped (staged) tile, and per-bin
-// counters.
-template <bool IN8, bool OUT8>
-struct RJPartSmem {
-    using F = RJFmt<IN8, OUT8>;
-    typename F::In in[RJ_STAGES][F::TILE];
-    typename F::Out stage[F::TILE];
-    typename F::Bin stage_bin[F::TILE];
-    unsigned hist[RJ_LMAX];
-    unsigned loff[RJ_LMAX];
-    unsigned long long gdelta[RJ_LMAX];  // output position of staged slot i = gdelta[bin] + i
-    uint64_t bar[RJ_STAGES];
-    RJTileRange info[RJ_STAGES];
-    unsigned warp_tot[32];
-    unsigned total;  // elements of the current tile (scan by warp 0)
-    long long split[2][RJ_SPLIT_MAX];  // range mode: the splitters of this tile and the next
-    int ok;
+// Shape of a partition kernel's CTA: worker threads, control warps, resident
+// CTAs per SM, input tiles in flight.  Chosen with the tile sizes
+// (radixpart.cuh) by measuring both passes of R 2^27 x S 2^30 (hash), the
+// learned and sampled MPSM join of 2^26 x 2^28 and the group-by of 2^27:
+//   16-byte in, packed out, hash     probe pass 1 4.79 ms.  One CTA per SM and
+//     the largest tile: a tile reserves one run per bin, and at 2048-tuple
+//     tiles the 64-bit atomics on 128 cursors alone took a third of the pass
+//     (7.7 ms; 5.1 ms with them taken out).  2 x 512 threads, 4096: 7.1 ms.
+//   packed in and out, hash          probe pass 2 4.03 ms.  256 bins: two
+//     control warps reserve four each per lane (one warp: 4.70 ms).
+//   model and range bins wait on their leaf and splitter loads and take
+//     whichever shape measured best: 3.00 and 1.77 ms (model), 3.92 and
+//     2.90 ms (range, unpacked), group-by 0.72 ms (hash, unpacked).
+// Against one kernel shape of 2 x 256 or 512 threads without control warps,
+// three barriers per tile and reservations waited for inside a tile: 6.78,
+// 4.66, 3.09, 1.95, 3.92, 3.05 and 0.81 ms.
+template <int WORKERS, int CONTROL, int CTAS, int STAGES>
+struct RJShapeOf {
+    static constexpr int T = WORKERS, NC = CONTROL, MINB = CTAS, ST = STAGES, THREADS = T + 32 * NC;
 };
-static_assert(2 * (sizeof(RJPartSmem<false, false>) + 1024) <= 233472, "two partition CTAs per SM");
-static_assert(2 * (sizeof(RJPartSmem<false, true>) + 1024) <= 233472, "two partition CTAs per SM");
-static_assert(2 * (sizeof(RJPartSmem<true, true>) + 1024) <= 233472, "two partition CTAs per SM");
+template <bool IN8, bool OUT8, int MODE>
+struct RJShape : RJShapeOf<480, 1, 2, 1> {};  // packed model and range passes; 16-byte tuples in and out
+template <>
+struct RJShape<true, true, RJ_MODE_HASH> : RJShapeOf<448, 2, 2, 1> {};
+template <>
+struct RJShape<false, true, RJ_MODE_HASH> : RJShapeOf<992, 1, 1, 1> {};
+template <>
+struct RJShape<false, true, RJ_MODE_MODEL> : RJShapeOf<992, 1, 1, 2> {};
+template <>
+struct RJShape<false, true, RJ_MODE_RANGE> : RJShapeOf<992, 1, 1, 2> {};
 
+// Shared memory of one partition CTA: a ring of input tiles that bulk
+// copies fill ahead of use, the grouped (staged) tile, and per-bin
+// counters.
+template <bool IN8, bool OUT8, int MODE>
+struct RJPartSmem {
+    using F = RJFmt<IN8, OUT8, MODE>;
+    // Model and range passes have at most 2^8 bins (RJ_SPLIT_MAX).
+    static constexpr int BINS = MODE == RJ_MODE_HASH ? RJ_LMAX : RJ_SPLIT_MAX;
+    static constexpr int ST = RJShape<IN8, OUT8, MODE>::ST;
+    typename F::In in[ST][F::TILE];
+    typename F::Out stage[F::TILE];
+    unsigned long long gdelta[BINS];  // output position of staged slot i = gdelta[bin] + i
+    unsigned hist[2][BINS];           // tile counts per bin; tiles alternate
+    unsigned loff[BINS];
+    typename F::Bin stage_bin[F::TILE];
+    uint64_t bar[ST];
+    RJTileRange info[ST];
+    unsigned total[2];                 // elements of a tile; tiles alternate
+    int seg;                           // the tile being reserved: its segment
+    unsigned hot;                      // a bin that held many of the last tile's tuples, else no bin
+    int ok;
+    long long split[2][MODE == RJ_MODE_RANGE ? RJ_SPLIT_MAX : 1];  // the splitters of this tile and the next
+};
 __device__ __forceinline__ unsigned rj_range_bin(const long long* sp, int n, long long k)
 {
     int lo = 0;
@@ -266,12 +298,11 @@ __device__ __forceinline__ unsigned rj_range_bin(const long long* sp, int n, lon
     return (unsigned)lo;
 }
 
-// All threads: the splitters of segment seg into dst.
-template <int THREADS>
-__device__ __forceinline__ void rj_load_split(const RJPass& a, long long* dst, int seg)
+// One warp: the splitters of segment seg into dst.
+__device__ __forceinline__ void rj_load_split(const RJPass& a, long long* dst, int seg, int lane)
 {
     const long long* src = a.split + (a.nseg > 1 ? ((long long)seg << a.lbits) : 0);
-    for (int i = threadIdx.x; i < a.nsplit; i += THREADS) dst[i] = src[i];
+    for (int i = lane; i < a.nsplit; i += 32) dst[i] = src[i];
 }
 
 // Histogram of range bins of in[0], in[step], ...: fine bin = coarse bin
@@ -306,263 +337,260 @@ __global__ void __launch_bounds__(1024) rj_hist_range_kernel(const longlong2* __
 // Packed tiles start at an even word (regions and tiles are even), and the
 // copy is rounded up to 16 bytes: at most one word past the tile, inside
 // the buffer's 16-byte tail, which is never used as data.
-template <bool IN8, bool OUT8>
-__device__ __forceinline__ void rj_issue_tile(const RJPass& a, RJPartSmem<IN8, OUT8>& sm, RJSegCursor& cur, int slot,
-                                              long long tile)
+template <bool IN8, bool OUT8, int MODE>
+__device__ __forceinline__ void rj_issue_tile(const RJPass& a, RJPartSmem<IN8, OUT8, MODE>& sm, RJSegCursor& cur,
+                                              int slot, long long tile)
 {
-    using F = RJFmt<IN8, OUT8>;
-    const RJTileRange r = rj_tile_range<F::TILE>(a, cur, tile);
+    using F = RJFmt<IN8, OUT8, MODE>;
+    const RJTileRange r = rj_tile_range(a, cur, tile);
     sm.info[slot] = r;
     const unsigned bytes = ((unsigned)(r.end - r.begin) * (unsigned)sizeof(typename F::In) + 15u) & ~15u;
     mbar_arrive_expect_tx(&sm.bar[slot], bytes);
     bulk_load(sm.in[slot], reinterpret_cast<const typename F::In*>(a.in) + r.begin, bytes, &sm.bar[slot]);
 }
 
-// How a pass computes a tuple's bin, fixed per kernel instance so that no
-// per-tuple branch chooses it.
-enum RJMode { RJ_MODE_HASH = 0, RJ_MODE_MODEL = 1, RJ_MODE_RANGE = 2 };
-
-// Threads of a partition CTA: 256 for hash bins of 16-byte tuples, 512
-// otherwise.  The learned model's bins and splitter searches wait on loads
-// (the key's leaf, the splitters) and measured faster with the larger CTA:
-// MPSM partition phase at theta 1.0, 8.05 against 7.18 ms (model) and 10.59
-// against 10.14 ms (sampled splitters) with 256 threads.
-template <bool IN8, int MODE>
-constexpr int rj_pt_threads()
-{
-    return (IN8 || MODE != RJ_MODE_HASH) ? RJ_PT_THREADS8 : RJ_PT_THREADS16;
-}
+// One partition pass.  T worker threads move the tuples; the control warps
+// make the global reservations, and the first of them also starts the input
+// copies and scans the bins, so that no worker waits on an atomic or holds
+// the others up with a scan.  Bound: the shared-memory traffic of ranking and
+// staging (about 25 wavefronts per 32 tuples) and the workers' instructions;
+// the probe side's passes of 2^27 x 2^30 move 5.4 and 4.3 TB/s.  Two tiles are in the works: while tile k waits for the
+// reservations of its runs, tile k + 1 is binned and ranked; while the
+// control warp scans the bins of tile k + 1, the workers write tile k out.
+// Two CTA barriers per tile:
+//   workers                                   control warps
+//   bin and rank tile k + 1                   reserve the runs of tile k
+//   -- barrier 1
+//   write out tile k                          next input copy; scan tile k + 1
+//   -- barrier 2
+//   group tile k + 1 in the stage             (reserve the runs of tile k + 1)
+static_assert(sizeof(RJPartSmem<false, true, RJ_MODE_HASH>) <= 232448, "one CTA per SM");
+static_assert(sizeof(RJPartSmem<false, true, RJ_MODE_MODEL>) <= 232448, "one CTA per SM");
+static_assert(2 * (sizeof(RJPartSmem<true, true, RJ_MODE_HASH>) + 1024) <= 233472, "two CTAs per SM");
+static_assert(2 * (sizeof(RJPartSmem<true, true, RJ_MODE_RANGE>) + 1024) <= 233472, "two CTAs per SM");
+static_assert(2 * (sizeof(RJPartSmem<false, false, RJ_MODE_HASH>) + 1024) <= 233472, "two CTAs per SM");
+static_assert(2 * (sizeof(RJPartSmem<false, false, RJ_MODE_RANGE>) + 1024) <= 233472, "two CTAs per SM");
 
 template <bool IN8, bool OUT8, int MODE>
-__global__ void __launch_bounds__(rj_pt_threads<IN8, MODE>(), PYG_RJ_PT_MINB) rj_partition_kernel(RJPass a, long long ntiles)
+__global__ void __launch_bounds__(RJShape<IN8, OUT8, MODE>::THREADS, RJShape<IN8, OUT8, MODE>::MINB)
+    rj_partition_kernel(RJPass a, long long ntiles)
 {
-    using F = RJFmt<IN8, OUT8>;
+    using F = RJFmt<IN8, OUT8, MODE>;
+    using Smem = RJPartSmem<IN8, OUT8, MODE>;
     using Out = typename F::Out;
     if (a.ntiles_dev) ntiles = (long long)*a.ntiles_dev;
     extern __shared__ __align__(128) unsigned char rj_pt_raw[];
-    RJPartSmem<IN8, OUT8>& sm = *reinterpret_cast<RJPartSmem<IN8, OUT8>*>(rj_pt_raw);
-    constexpr int T = rj_pt_threads<IN8, MODE>();
+    Smem& sm = *reinterpret_cast<Smem*>(rj_pt_raw);
+    constexpr int T = RJShape<IN8, OUT8, MODE>::T;
+    constexpr int NC = RJShape<IN8, OUT8, MODE>::NC;
     constexpr int PER = F::TILE / T;
+    constexpr int ST = Smem::ST;
+    constexpr int BINS = Smem::BINS;
+    static_assert(PER * T == F::TILE, "whole rows of elements");
     const int L = 1 << a.lbits;
-    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    Out* out = reinterpret_cast<Out*>(a.out);
-    bool miss = false;  // a 16-byte tuple outside the packed frame
-    RJSegCursor segc{-1, -1, -1, 0, 0};  // thread 0: segment of the tiles it issues
-    for (int b = tid; b < RJ_LMAX; b += T) sm.hist[b] = 0;
-    if (tid == 0) {
-        for (int s = 0; s < RJ_STAGES; ++s) mbar_init(&sm.bar[s], 1);
-        mbar_fence_init();
-        for (int s = 0; s < RJ_STAGES; ++s)
-            if (blockIdx.x + (long long)s * gridDim.x < ntiles)
-                rj_issue_tile(a, sm, segc, s, blockIdx.x + (long long)s * gridDim.x);
-        sm.ok = 1;
-    }
-    __syncthreads();
-    if (a.nsplit) {
-        rj_load_split<T>(a, sm.split[0], sm.info[0].seg);
-        __syncthreads();
-    }
-    long long k = 0;
-    for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++k) {
-        const int slot = (int)(k % RJ_STAGES);
-        const unsigned parity = (unsigned)((k / RJ_STAGES) & 1);
-        // Every thread waits for the tile; a wait that runs out marks the
-        // CTA failed and that thread's tuples are left out, so nothing is
-        // written from memory the copy did not fill.
-        const bool landed = mbar_wait(&sm.bar[slot], parity, kBulkWaitNs);
-        if (!landed) sm.ok = 0;
-        const RJTileRange cur = sm.info[slot];
-        const unsigned n = (unsigned)(cur.end - cur.begin);
-        // (1) Bin and rank every tuple; one shared atomic per (warp, bin).
-        Out t[PER];
-        unsigned bin[PER], rank[PER];
-        auto bin_rank = [&](int j, bool valid) {
-            const unsigned i = j * T + tid;
-            bin[j] = 0xFFFFFFFFu;
-            if (valid) {
-                const typename F::In e = sm.in[slot][i];
-                const long long key = rj_key(e, a.kbase);
-                if constexpr (IN8 || !OUT8) {
-                    t[j] = e;
-                } else {
-                    // Pack: (key - kbase) | (payload - pbase) << 32.
-                    const unsigned long long dk = (unsigned long long)e.x - a.kbase;
-                    const unsigned long long dp = (unsigned long long)e.y - a.pbase;
-                    miss |= ((dk | dp) >> 32) != 0;
-                    t[j] = (dk & 0xFFFFFFFFULL) | (dp << 32);
-                }
-                // 16-byte passes test nsplit at run time, the hash instance
-                // too (it never has splitters): compiled without the test,
-                // the first pass of the 2^30-tuple probe side measured 7.51
-                // against 6.95 ms.
-                if constexpr (MODE == RJ_MODE_MODEL)
-                    bin[j] = rj_bin(rj_model_code(a.model, key), a.shift, a.mask);
-                else if constexpr (!IN8)
-                    bin[j] = a.nsplit ? rj_range_bin(sm.split[a.nseg > 1 ? (k & 1) : 0], a.nsplit, key)
-                                      : rj_bin(rj_hash((uint64_t)key), a.shift, a.mask);
-                else if constexpr (MODE == RJ_MODE_RANGE)
-                    bin[j] = rj_range_bin(sm.split[a.nseg > 1 ? (k & 1) : 0], a.nsplit, key);
-                else
-                    bin[j] = rj_bin(rj_hash((uint64_t)key), a.shift, a.mask);
-            }
-            // Skewed keys put many lanes of a warp into one bin: when at
-            // least 8 lanes share lane 0's bin, they take their ranks from
-            // one atomic (lane order), the others one atomic each.
-            const unsigned b0 = __shfl_sync(0xffffffffu, bin[j], 0);
-            const unsigned m0 = __ballot_sync(0xffffffffu, valid && bin[j] == b0);
-            if (__popc(m0) >= 8) {
-                unsigned base = 0;
-                if (lane == 0) base = atomicAdd(&sm.hist[b0], (unsigned)__popc(m0));
-                base = __shfl_sync(0xffffffffu, base, 0);
-                if ((m0 >> lane) & 1) rank[j] = base + __popc(m0 & ((1u << lane) - 1u));
-                else if (valid) rank[j] = atomicAdd(&sm.hist[bin[j]], 1u);
-            } else if (valid) {
-                rank[j] = atomicAdd(&sm.hist[bin[j]], 1u);
-            }
-        };
-        // Packed passes: full tiles (all but the last of each segment) skip
-        // the per-tuple bounds test (second pass of the 2^30-tuple probe side
-        // 4.94 -> 4.68 ms).  16-byte passes keep one loop: there the second
-        // copy of the loop measured slower (7.03 -> 8.15 ms; 127 registers).
-        if (IN8 && landed && n == (unsigned)F::TILE) {
-#pragma unroll
-            for (int j = 0; j < PER; ++j) bin_rank(j, true);
-        } else {
-#pragma unroll
-            for (int j = 0; j < PER; ++j) bin_rank(j, landed && j * T + tid < n);
+    const int tid = threadIdx.x, lane = tid & 31;
+    for (int b = tid; b < 2 * BINS; b += T + 32 * NC) (&sm.hist[0][0])[b] = 0;
+    if (tid >= T) {
+        // ---- control warps; the first one does all but the reservations
+        const int ct = tid - T;
+        const bool first = ct < 32;
+        RJSegCursor segc{-1, -1, -1, 0, 0};  // lane 0: segment of the tiles it issues
+        if (ct == 0) {
+            for (int s = 0; s < ST; ++s) mbar_init(&sm.bar[s], 1);
+            mbar_fence_init();
+            for (int s = 0; s < ST; ++s)
+                if (blockIdx.x + (long long)s * gridDim.x < ntiles)
+                    rj_issue_tile(a, sm, segc, s, blockIdx.x + (long long)s * gridDim.x);
+            sm.ok = 1;
+            sm.hot = ~0u;
+            sm.total[0] = sm.total[1] = 0;
         }
-        __syncthreads();  // A: histogram complete
-        if (!sm.ok) break;
-        // (2) In-tile offsets of the bins, reservation of each non-empty
-        // bin's run (one global atomic) and reset of its counter.  Thread
-        // tid handles bins tid + q x T.  With a thread per bin (packed
-        // passes, 512 threads) the whole CTA scans; with fewer threads than
-        // bins (16-byte passes, 256 threads) warp 0 scans alone and the
-        // others go on to barrier C: measured 6.9 against 12.7 ms for the
-        // 2^30-tuple probe side's first pass (one barrier fewer per tile,
-        // where only 16 warps share an SM).
-        constexpr int BPT = (RJ_LMAX + T - 1) / T;
-        unsigned c[BPT], ex[BPT], total;
-        // The reservation's result (a global atomic, about a microsecond
-        // away) is first needed after the tile is staged.
-        unsigned long long resv[BPT], bstart[BPT], bcap[BPT];
-        auto reserve = [&](int q) {
-            const int b = tid + q * T;
-            resv[q] = 0;
-            bstart[q] = 0;
-            bcap[q] = ~0ULL;
-            if (b < L) {
-                if (c[q]) {
-                    const unsigned ob = ((unsigned)cur.seg << a.lbits) | (unsigned)b;
-                    bstart[q] = a.bin_start[ob];
-                    if (a.bin_cap) bcap[q] = a.bin_cap[ob];
-                    resv[q] = atomicAdd(&a.cursor[ob], (unsigned long long)c[q]);
+        __syncwarp();
+        if constexpr (MODE == RJ_MODE_RANGE) {
+            if (first && blockIdx.x < ntiles) rj_load_split(a, sm.split[0], sm.info[0].seg, lane);
+        }
+        __syncthreads();
+        long long k = 0;
+        for (long long tile = blockIdx.x;; tile += gridDim.x, ++k) {
+            __syncthreads();  // 1
+            if (!sm.ok || tile >= ntiles) break;
+            const int slot = (int)(k % ST);
+            unsigned* hist = sm.hist[k & 1];
+            if (first) {
+                __syncwarp();
+                if (lane == 0) {
+                    sm.seg = sm.info[slot].seg;
+                    const long long nt = tile + (long long)ST * gridDim.x;
+                    if (nt < ntiles) {
+                        fence_proxy_async_smem();
+                        rj_issue_tile(a, sm, segc, slot, nt);
+                    }
                 }
-                sm.hist[b] = 0;
-            }
-        };
-        if constexpr (BPT == 1) {
-            c[0] = tid < L ? sm.hist[tid] : 0u;
-            unsigned incl = c[0];
+                // Range mode over several segments: the next tile's splitters
+                // (its copy has been issued, so its segment is known).
+                if constexpr (MODE == RJ_MODE_RANGE) {
+                    __syncwarp();
+                    if (a.nseg > 1 && tile + gridDim.x < ntiles)
+                        rj_load_split(a, sm.split[(k + 1) & 1], sm.info[(k + 1) % ST].seg, lane);
+                }
+                // Scan of the bins: lane l holds the 4 G consecutive ones from
+                // 4 G l (G = 1 below 128 bins).
+                const uint4* h4 = reinterpret_cast<const uint4*>(hist);
+                uint4* l4 = reinterpret_cast<uint4*>(sm.loff);
+                constexpr int GMAX = BINS / 128;
+                const int G = L > 128 ? L >> 7 : 1;
+                uint4 h[GMAX];
+                unsigned sum = 0, top = 0;
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                unsigned v = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += v;
-            }
-            if (lane == 31) sm.warp_tot[w] = incl;
-            __syncthreads();  // B
-            // Prefix over the warp totals, by one more shuffle scan per warp.
-            constexpr int NW = T / 32;
-            const unsigned wt = lane < NW ? sm.warp_tot[lane] : 0u;
-            unsigned wincl = wt;
-#pragma unroll
-            for (int o = 1; o < NW; o <<= 1) {
-                const unsigned v = __shfl_up_sync(0xffffffffu, wincl, o);
-                if (lane >= o) wincl += v;
-            }
-            ex[0] = incl - c[0] + __shfl_sync(0xffffffffu, wincl - wt, w);
-            total = __shfl_sync(0xffffffffu, wincl, NW - 1);
-            if (tid < L) sm.loff[tid] = ex[0];
-            reserve(0);
-            __syncthreads();  // C: in-tile offsets ready
-        } else {
-            // Lane l of warp 0 owns the PB consecutive bins from l x PB.
-            if (w == 0) {
-                const int PB = (L + 31) >> 5;
-                const int b0 = lane * PB;
-                unsigned sum = 0;
-                for (int q = 0; q < PB; ++q)
-                    if (b0 + q < L) sum += sm.hist[b0 + q];
-                unsigned incl = sum;
+                for (int g = 0; g < GMAX; ++g) {
+                    const int b = 4 * (G * lane + g);
+                    h[g] = g < G && b < L ? h4[b >> 2] : make_uint4(0, 0, 0, 0);
+                    sum += h[g].x + h[g].y + h[g].z + h[g].w;
+                    top = max(top, max(max(h[g].x << 9 | b, h[g].y << 9 | (b + 1)),
+                                       max(h[g].z << 9 | (b + 2), h[g].w << 9 | (b + 3))));
+                }
+                unsigned run = sum;
 #pragma unroll
                 for (int o = 1; o < 32; o <<= 1) {
-                    const unsigned v = __shfl_up_sync(0xffffffffu, incl, o);
-                    if (lane >= o) incl += v;
+                    const unsigned v = __shfl_up_sync(0xffffffffu, run, o);
+                    if (lane >= o) run += v;
                 }
-                unsigned run = incl - sum;
-                for (int q = 0; q < PB; ++q)
-                    if (b0 + q < L) {
-                        sm.loff[b0 + q] = run;
-                        run += sm.hist[b0 + q];
-                    }
-                if (lane == 31) sm.total = incl;
-            }
-            __syncthreads();  // C: in-tile offsets ready
-            total = sm.total;
+                unsigned x = run - sum;
 #pragma unroll
-            for (int q = 0; q < BPT; ++q) {
-                const int b = tid + q * T;
-                c[q] = b < L ? sm.hist[b] : 0u;
-                ex[q] = b < L ? sm.loff[b] : 0u;
-                reserve(q);
+                for (int g = 0; g < GMAX; ++g) {
+                    const int b = 4 * (G * lane + g);
+                    if (g < G && b < L) l4[b >> 2] = make_uint4(x, x + h[g].x, x + h[g].x + h[g].y, x + h[g].x + h[g].y + h[g].z);
+                    x += h[g].x + h[g].y + h[g].z + h[g].w;
+                }
+                top = __reduce_max_sync(0xffffffffu, top);
+                if (lane == 31) {
+                    sm.total[k & 1] = run;
+                    sm.hot = (top >> 9) * 4 >= (unsigned)a.tile ? top & 511u : ~0u;
+                }
+            }
+            __syncthreads();  // 2
+            const int seg = sm.seg;
+            // Each non-empty bin reserves its run with one global atomic and
+            // its counter is reset.  A run that outgrows its region goes to
+            // the dump; the host redoes the relation from an exact histogram.
+            constexpr int CT = 32 * NC, U = BINS / CT < 4 ? BINS / CT : 4;
+            for (int b0 = ct; b0 < L; b0 += CT * U) {
+                unsigned c[U];
+                unsigned long long pos[U], end[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int b = b0 + u * CT;
+                    c[u] = b < L ? hist[b] : 0u;
+                    if (c[u]) {
+                        const unsigned ob = ((unsigned)seg << a.lbits) | (unsigned)b;
+                        const unsigned long long start = a.bin_start[ob];
+                        end[u] = a.bin_cap ? start + a.bin_cap[ob] : ~0ULL;
+                        pos[u] = start + atomicAdd(&a.cursor[(size_t)ob * a.cstride], (unsigned long long)c[u]);
+                        hist[b] = 0;
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int b = b0 + u * CT;
+                    if (c[u]) {
+                        const bool over = pos[u] + c[u] > end[u];
+                        if (over) atomicOr(a.ovf, 1u);
+                        sm.gdelta[b] = (over ? a.dump : pos[u]) - sm.loff[b];
+                    }
+                }
             }
         }
-        // (3) Group the tile by bin in shared memory.
+        if (ct == 0 && !sm.ok) atomicOr(a.err, 1u);
+        return;
+    }
+    // ---- workers
+    Out* out = reinterpret_cast<Out*>(a.out);
+    unsigned miss = 0;  // high halves of packed offsets: nonzero when a tuple was outside the frame
+    __syncthreads();
+    long long k = 0;
+    for (long long tile = blockIdx.x;; tile += gridDim.x, ++k) {
+        const bool more = tile < ntiles;  // uniform; the last turn only writes out
+        Out t[PER];
+        unsigned br[PER];  // bin << 16 | rank
+        if (more) {
+            const int slot = (int)(k % ST);
+            unsigned* hist = sm.hist[k & 1];
+            // Every thread waits for the tile; a wait that runs out marks the
+            // CTA failed and that thread's tuples are left out, so nothing is
+            // written from memory the copy did not fill.
+            const bool landed = mbar_wait(&sm.bar[slot], (unsigned)((k / ST) & 1), kBulkWaitNs);
+            if (!landed) sm.ok = 0;
+            const unsigned n = landed ? (unsigned)(sm.info[slot].end - sm.info[slot].begin) : 0u;
+            const unsigned hot = sm.hot;
+            // Bin and rank every tuple with a shared atomic.  When one bin
+            // held at least a quarter of the last tile (skewed keys), the
+            // lanes of that bin take their ranks from one atomic.
+            auto bin_rank = [&](int j, bool valid) {
+                br[j] = 0xFFFFFFFFu;
+                unsigned bin = 0;
+                if (valid) {
+                    const typename F::In e = sm.in[slot][j * T + tid];
+                    const long long key = rj_key(e, a.kbase);
+                    if constexpr (IN8 || !OUT8) {
+                        t[j] = e;
+                    } else {
+                        // Pack: (key - kbase) | (payload - pbase) << 32.
+                        const unsigned long long dk = (unsigned long long)e.x - a.kbase;
+                        const unsigned long long dp = (unsigned long long)e.y - a.pbase;
+                        miss |= (unsigned)(dk >> 32) | (unsigned)(dp >> 32);
+                        t[j] = (dk & 0xFFFFFFFFULL) | (dp << 32);
+                    }
+                    if constexpr (MODE == RJ_MODE_MODEL)
+                        bin = rj_bin(rj_model_code(a.model, key), a.shift, a.mask);
+                    else if constexpr (MODE == RJ_MODE_RANGE)
+                        bin = rj_range_bin(sm.split[a.nseg > 1 ? (k & 1) : 0], a.nsplit, key);
+                    else
+                        bin = rj_bin(rj_hash((uint64_t)key), a.shift, a.mask);
+                }
+                if (hot != ~0u) {
+                    const unsigned m = __ballot_sync(0xffffffffu, valid && bin == hot);
+                    unsigned base = 0;
+                    if (m) {
+                        const int lead = __ffs(m) - 1;
+                        if (lane == lead) base = atomicAdd(&hist[hot], (unsigned)__popc(m));
+                        base = __shfl_sync(0xffffffffu, base, lead);
+                    }
+                    if (valid)
+                        br[j] = (bin << 16) | (bin == hot ? base + __popc(m & ((1u << lane) - 1u)) : atomicAdd(&hist[bin], 1u));
+                } else if (valid) {
+                    br[j] = (bin << 16) | atomicAdd(&hist[bin], 1u);
+                }
+            };
+            if (IN8 && n == (unsigned)F::TILE) {
+#pragma unroll
+                for (int j = 0; j < PER; ++j) bin_rank(j, true);
+            } else {
+#pragma unroll
+                for (int j = 0; j < PER; ++j) bin_rank(j, j * T + tid < n);
+            }
+        }
+        __syncthreads();  // 1: hist[k] complete, ring slot consumed; stage and gdelta of the tile before complete
+        if (!sm.ok) break;
+        if (k > 0) {
+            // Write the staged tile, each bin's run contiguously.
+            const unsigned total = sm.total[(k & 1) ^ 1];
+#pragma unroll
+            for (int j = 0; j < PER; ++j) {
+                const unsigned i = j * T + tid;
+                if (i < total) __stcs(&out[sm.gdelta[sm.stage_bin[i]] + i], sm.stage[i]);
+            }
+        }
+        if (!more) break;
+        __syncthreads();  // 2: in-tile offsets ready, the stage is free
 #pragma unroll
         for (int j = 0; j < PER; ++j)
-            if (bin[j] != 0xFFFFFFFFu) {
-                const unsigned s = sm.loff[bin[j]] + rank[j];
+            if (br[j] != 0xFFFFFFFFu) {
+                const unsigned bin = br[j] >> 16;
+                const unsigned s = sm.loff[bin] + (br[j] & 0xFFFFu);
                 sm.stage[s] = t[j];
-                sm.stage_bin[s] = (typename F::Bin)bin[j];
+                sm.stage_bin[s] = (typename F::Bin)bin;
             }
-        // Range mode over several segments: the next tile's splitters
-        // (its copy was issued a tile ago, so its segment is known).
-        if (a.nsplit && a.nseg > 1 && tile + gridDim.x < ntiles)
-            rj_load_split<T>(a, sm.split[(k + 1) & 1], sm.info[(k + 1) % RJ_STAGES].seg);
-        // Per bin, the output position of staged slot i is gdelta + i.
-#pragma unroll
-        for (int q = 0; q < BPT; ++q) {
-            const int b = tid + q * T;
-            if (b < L && c[q]) {
-                unsigned long long gd = bstart[q] + resv[q] - ex[q];
-                if (resv[q] + c[q] > bcap[q]) {  // outgrew its region: not written; the host redoes the pass exactly
-                    atomicOr(a.ovf, 1u);
-                    gd = kSkipRun;
-                }
-                sm.gdelta[b] = gd;
-            }
-        }
-        __syncthreads();  // D: ring slot consumed, stage and global offsets complete
-        if (tid == 0) {
-            const long long nt = tile + (long long)RJ_STAGES * gridDim.x;
-            if (nt < ntiles) {
-                fence_proxy_async_smem();
-                rj_issue_tile(a, sm, segc, slot, nt);
-            }
-        }
-        // (4) Write each bin's run contiguously (total <= PER x T: PER
-        // unrolled steps cover the tile and their loads overlap).
-#pragma unroll
-        for (int j = 0; j < PER; ++j) {
-            const unsigned i = j * T + tid;
-            if (i < total) {
-                const unsigned long long gd = sm.gdelta[sm.stage_bin[i]];
-                if (gd != kSkipRun) __stcs(&out[gd + i], sm.stage[i]);
-            }
-        }
     }
-    __syncthreads();
-    if (tid == 0 && !sm.ok) atomicOr(a.err, 1u);
     if (miss) atomicOr(a.frame, 1u);
 }
 
@@ -573,10 +601,10 @@ template <bool IN8, bool OUT8, int MODE>
 int launch_pass_t(pyg_ctx* ctx, const RJPass& p, long long ntiles)
 {
     auto fn = rj_partition_kernel<IN8, OUT8, MODE>;
-    const size_t smem = sizeof(RJPartSmem<IN8, OUT8>);
+    const size_t smem = sizeof(RJPartSmem<IN8, OUT8, MODE>);
     PYG_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
-    constexpr int T = rj_pt_threads<IN8, MODE>();
+    constexpr int T = RJShape<IN8, OUT8, MODE>::THREADS;
     PYG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, T, smem));
     if (per_sm < 1) per_sm = 1;
     long long grid = std::min<long long>(ntiles, (long long)ctx->sm_count * per_sm);
@@ -609,8 +637,16 @@ int launch_pass(pyg_ctx* ctx, const RJPass& p, long long ntiles, bool in8, bool 
 
 }  // namespace
 
-void layout_exact(const std::vector<unsigned long long>& h, int C, int sub, RJLayout& L, bool pack)
+static void layout_tiles(RJLayout& L, int64_t n, bool pack, bool model)
 {
+    L.tile1 = rj_tile(!pack ? RJ_TILE_U : (model ? RJ_TILE_PM : RJ_TILE_P), n);
+    L.tile2 = rj_tile(!pack ? RJ_TILE_U : (model ? RJ_TILE_8M : RJ_TILE_8), n);
+}
+
+void layout_exact(const std::vector<unsigned long long>& h, int64_t n, int C, int sub, RJLayout& L, bool pack,
+                  bool model)
+{
+    layout_tiles(L, n, pack, model);
     const size_t F = h.size();
     L.sampled = false;
     L.packed = pack;
@@ -631,11 +667,11 @@ void layout_exact(const std::vector<unsigned long long>& h, int C, int sub, RJLa
         L.tiles2_max = 0;
         for (int c = 0; c < C; ++c) {
             L.ccap[c] = L.cstart[c + 1] - L.cstart[c];
-            L.tiles2_max += (L.ccap[c] + RJ_TILE8 - 1) / RJ_TILE8;
+            L.tiles2_max += (L.ccap[c] + L.tile2 - 1) / L.tile2;
         }
     } else {
         for (int c = 0; c < C; ++c)
-            L.tiles2[c + 1] = L.tiles2[c] + (L.cstart[c + 1] - L.cstart[c] + RJ_TILE - 1) / RJ_TILE;
+            L.tiles2[c + 1] = L.tiles2[c] + (L.cstart[c + 1] - L.cstart[c] + L.tile2 - 1) / L.tile2;
         L.tiles2_max = L.tiles2[C];
     }
     L.count = h;
@@ -648,14 +684,14 @@ unsigned long long sampled_cap(unsigned long long c, long long step, unsigned lo
     return (unsigned long long)std::ceil((x + 6.0 * std::sqrt(x) + 8.0) * (double)step) + extra;
 }
 
-void layout_sampled(const std::vector<unsigned long long>& sc, long long step, int C, int sub, RJLayout& L,
-                    bool pack)
+void layout_sampled(const std::vector<unsigned long long>& sc, long long step, int64_t n, int C, int sub, RJLayout& L,
+                    bool pack, bool model)
 {
+    layout_tiles(L, n, pack, model);
     const size_t F = sc.size();
     L.sampled = true;
     L.packed = pack;
     auto sz = [&](unsigned long long c) { return pack ? (c + 1) & ~1ULL : c; };
-    const int tile2 = pack ? RJ_TILE8 : RJ_TILE;
     L.fcap.assign(F, 0);
     L.fstart.assign(F + 1, 0);
     for (size_t f = 0; f < F; ++f) {
@@ -670,7 +706,7 @@ void layout_sampled(const std::vector<unsigned long long>& sc, long long step, i
         for (size_t f = (size_t)c << sub; f < (size_t)(c + 1) << sub; ++f) cc += sc[f];
         L.ccap[c] = sz(sampled_cap(cc, step, 1024));
         L.cstart[c + 1] = L.cstart[c] + L.ccap[c];
-        L.tiles2_max += (L.ccap[c] + tile2 - 1) / tile2;
+        L.tiles2_max += (L.ccap[c] + L.tile2 - 1) / L.tile2;
     }
     L.tiles2.clear();
     L.count.clear();
@@ -726,8 +762,8 @@ int upload_layout(pyg_ctx* ctx, const RJLayout& L, const RJSideDev& d, int F, in
     } else if ((rc = stage_h2d(ctx, d.tiles2, L.tiles2.data(), (size_t)(C + 1) * 8))) {
         return rc;
     }
-    PYG_CUDA(cudaMemsetAsync(d.cur1, 0, (size_t)(C + F) * 8, ctx->stream));  // cur1 and cur2 are adjacent
-    const unsigned long long w[4] = {0, (unsigned long long)n, 0, (unsigned long long)((n + RJ_TILE - 1) / RJ_TILE)};
+    PYG_CUDA(cudaMemsetAsync(d.cur1, 0, ((size_t)C * RJ_CURSOR_STRIDE + F) * 8, ctx->stream));  // cur1 and cur2 are adjacent
+    const unsigned long long w[4] = {0, (unsigned long long)n, 0, (unsigned long long)((n + L.tile1 - 1) / L.tile1)};
     return stage_h2d(ctx, d.whole, w, sizeof(w));
 }
 
@@ -748,12 +784,15 @@ int run_passes(pyg_ctx* ctx, const longlong2* in, int64_t n, const RJLayout& L, 
     p.seg_start = d.whole;
     p.seg_tile0 = d.wtiles;
     p.nseg = 1;
+    p.tile = L.tile1;
     p.shift = 64 - CB;
     p.mask = (unsigned)(C - 1);
     p.lbits = CB;
     p.bin_start = two ? d.cstart : d.fstart;
     p.bin_cap = L.sampled ? (two ? d.ccap : d.fcap) : nullptr;
-    p.cursor = two ? d.cur1 : d.cur2;
+    p.cursor = d.cur1;
+    p.cstride = RJ_CURSOR_STRIDE;
+    p.dump = two ? L.p1 : L.p2;
     p.err = err;
     p.ovf = ovf;
     p.kbase = L.kbase;
@@ -764,17 +803,17 @@ int run_passes(pyg_ctx* ctx, const longlong2* in, int64_t n, const RJLayout& L, 
         p.split = csplit;
         p.nsplit = C - 1;
     }
-    int rc = launch_pass(ctx, p, (n + RJ_TILE - 1) / RJ_TILE, false, L.packed);
+    int rc = launch_pass(ctx, p, (n + L.tile1 - 1) / L.tile1, false, L.packed);
     if (rc || !two) return rc;
     if (between) cudaEventRecord(between, ctx->stream);
     long long ntiles2;
     if (L.sampled || L.packed) {
         // Second-pass segments are the first pass's regions, filled to the
         // counts its cursors reached; the tile prefix is formed on the device.
-        rj_tile_prefix_kernel<<<1, 32, 0, ctx->stream>>>(d.cur1, d.ccap, C, L.packed ? RJ_TILE8 : RJ_TILE,
-                                                          d.tiles2);
+        rj_tile_prefix_kernel<<<1, 32, 0, ctx->stream>>>(d.cur1, RJ_CURSOR_STRIDE, d.count1, d.ccap, C,
+                                                          L.tile2, d.tiles2);
         PYG_LAUNCHED(ctx);
-        p.seg_count = d.cur1;
+        p.seg_count = d.count1;
         p.ntiles_dev = d.tiles2 + C;
         ntiles2 = (long long)L.tiles2_max;
     } else {
@@ -785,12 +824,15 @@ int run_passes(pyg_ctx* ctx, const longlong2* in, int64_t n, const RJLayout& L, 
     p.seg_start = d.cstart;
     p.seg_tile0 = d.tiles2;
     p.nseg = C;
+    p.tile = L.tile2;
     p.shift = 64 - FB;
     p.mask = (unsigned)((1 << sub) - 1);
     p.lbits = sub;
     p.bin_start = d.fstart;
     p.bin_cap = L.sampled ? d.fcap : nullptr;
     p.cursor = d.cur2;
+    p.cstride = 1;
+    p.dump = L.p2;
     if (fsplit) {
         p.split = fsplit;
         p.nsplit = (1 << sub) - 1;
@@ -901,8 +943,8 @@ int rp_partition_sides(pyg_ctx* ctx, RPSide* sd, int ns, int FB, bool two, unsig
         CBs[s] = coarse_bits(pack);
         const int C = 1 << CBs[s], sub = FB - CBs[s];
         std::vector<unsigned long long> hv(h, h + F);
-        if (exact) layout_exact(hv, C, sub, L, pack);
-        else layout_sampled(hv, st, C, sub, L, pack);
+        if (exact) layout_exact(hv, sd[s].n, C, sub, L, pack, sd[s].model != nullptr);
+        else layout_sampled(hv, st, sd[s].n, C, sub, L, pack, sd[s].model != nullptr);
         d[s].carve(meta + (size_t)s * per, F, C);
     };
     auto launch = [&](int s) {

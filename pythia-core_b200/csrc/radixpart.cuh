@@ -9,10 +9,10 @@
 //               of slack; a region that overflows is reported and the caller
 //               redoes the side exactly).
 //   passes      one tile pass (<= 9 bits) or two (coarse bits, then the rest
-//               inside each coarse partition).  A CTA receives 2048-tuple
-//               tiles by bulk copy into a two-deep shared-memory ring, groups
-//               a tile by bin in shared memory and writes each bin's run
-//               contiguously after one global reservation per (tile, bin).
+//               inside each coarse partition).  A CTA receives tiles of a few
+//               thousand tuples by bulk copy, groups a tile by bin in shared
+//               memory and writes each bin's run contiguously after one
+//               global reservation per (tile, bin).
 //   packing     (callers that opt in) when the histogram's reading of the
 //               relation shows that key - kbase and payload - pbase both
 //               fit in 32 bits for some frame (kbase, pbase), the passes
@@ -34,23 +34,23 @@ typedef struct pyg_cdf pyg_cdf;
 
 namespace pyg {
 
-#ifndef PYG_RJ_TILE
-#define PYG_RJ_TILE 2048
-#endif
-#ifndef PYG_RJ_PT_THREADS16
-#define PYG_RJ_PT_THREADS16 256
-#endif
-#ifndef PYG_RJ_PT_THREADS8
-#define PYG_RJ_PT_THREADS8 512
-#endif
-constexpr int RJ_TILE = PYG_RJ_TILE;            // tuples per partition tile
-constexpr int RJ_TILE8 = 4096;                  // packed words per partition tile (packed input)
-// Partition CTA threads: passes over 16-byte tuples run 8 tuples per thread
-// (fewer per-tile steps per tuple; measured 6.9 against 8.0 ms with 512
-// threads on the 2^30-tuple probe side), passes over packed words 8 words
-// per thread at 512 threads (4.99 against 5.73 ms with 256).
-constexpr int RJ_PT_THREADS16 = PYG_RJ_PT_THREADS16;
-constexpr int RJ_PT_THREADS8 = PYG_RJ_PT_THREADS8;
+// Largest tiles (elements) of a partition pass by what it reads and writes
+// (the kernels' shapes are in radixpart.cu).
+constexpr int RJ_TILE_U = 2400;    // 16-byte tuples in and out
+constexpr int RJ_TILE_P = 7936;    // 16-byte tuples in, packed words out: hash bins
+constexpr int RJ_TILE_PM = 3968;   //   model and range bins
+constexpr int RJ_TILE_8 = 5376;    // packed words in and out: hash bins
+constexpr int RJ_TILE_8M = 4800;   //   model and range bins
+constexpr int RJ_TILE_MIN = 1024;
+// Tile of a pass over n elements: the largest, halved until a pass has about
+// two tiles for each of 148 SMs (small relations would otherwise leave SMs
+// without a tile).
+inline int rj_tile(int largest, int64_t n)
+{
+    int t = largest;
+    while (t > RJ_TILE_MIN && n < (int64_t)t * 296) t = (t >> 1) & ~1;  // even: tiles of packed words start 16-byte aligned
+    return t;
+}
 constexpr int RJ_MAX_LOCAL_BITS = 9;     // bins of one partition pass
 constexpr int RJ_LMAX = 1 << RJ_MAX_LOCAL_BITS;
 constexpr int RJ_SPLIT_MAX = 256;        // range mode: splitters per pass segment (<= 2^8 bins)
@@ -150,16 +150,19 @@ struct RJLayout {
     std::vector<unsigned long long> tiles2;  // C + 1 tile prefix of the second pass (exact)
     std::vector<unsigned long long> count;   // F tuples per fine partition, once known
     unsigned long long p1 = 0, p2 = 0;       // tuples in the pass-1 / pass-2 buffers
+    int tile1 = 0, tile2 = 0;                // elements per tile of either pass
     unsigned long long tiles2_max = 0;       // upper bound of the second pass's tiles (sampled)
 };
 
-// Exact layout from exact per-fine-partition counts h (F = h.size()).
+// Exact layout of n tuples from exact per-fine-partition counts h (F = h.size()).
 // pack: regions rounded up to an even number of words (packed layouts).
-void layout_exact(const std::vector<unsigned long long>& h, int C, int sub, RJLayout& L, bool pack = false);
+// model: the passes' bins are a learned model's.
+void layout_exact(const std::vector<unsigned long long>& h, int64_t n, int C, int sub, RJLayout& L,
+                  bool pack = false, bool model = false);
 // Sampled layout from the counts sc of every step-th tuple: each region is
 // sized with six standard deviations of slack.
-void layout_sampled(const std::vector<unsigned long long>& sc, long long step, int C, int sub, RJLayout& L,
-                    bool pack = false);
+void layout_sampled(const std::vector<unsigned long long>& sc, long long step, int64_t n, int C, int sub, RJLayout& L,
+                    bool pack = false, bool model = false);
 // Frame of a packed layout from the key and payload ranges seen by the
 // histogram ([kmin, kmax], [pmin, pmax], signed).  exact: the ranges cover
 // every tuple; else they come from a sample and must leave a margin of at
@@ -174,10 +177,18 @@ bool common_key_frame(const long long* mm0, bool exact0, const long long* mm1, b
 // Bytes of one intermediate element of a layout.
 inline int elem_bytes(const RJLayout& L) { return L.packed ? 8 : 16; }
 
+// The first pass's cursors lie 128 bytes apart: 64-bit atomics on one line
+// are served one after another, and a tile's reservations are otherwise a
+// few lines that every CTA hits at once.
+constexpr int RJ_CURSOR_STRIDE = 16;
+
 // Device copy of one relation's partition metadata (u64 words).
 struct RJSideDev {
-    unsigned long long *fstart, *fcap, *cstart, *ccap, *cur1, *cur2, *tiles2, *whole, *wtiles;
-    static size_t words(int F, int C) { return (size_t)(F + 1) + F + (C + 1) + C + C + F + (C + 1) + 4; }
+    unsigned long long *fstart, *fcap, *cstart, *ccap, *cur1, *cur2, *count1, *tiles2, *whole, *wtiles;
+    static size_t words(int F, int C)
+    {
+        return (size_t)(F + 1) + F + (C + 1) + C + (size_t)C * RJ_CURSOR_STRIDE + F + C + (C + 1) + 4;
+    }
     void carve(unsigned long long* m, int F, int C)
     {
         fstart = m;
@@ -185,8 +196,9 @@ struct RJSideDev {
         cstart = fcap + F;
         ccap = cstart + C + 1;
         cur1 = ccap + C;
-        cur2 = cur1 + C;
-        tiles2 = cur2 + F;
+        cur2 = cur1 + (size_t)C * RJ_CURSOR_STRIDE;
+        count1 = cur2 + F;
+        tiles2 = count1 + C;
         whole = tiles2 + C + 1;
         wtiles = whole + 2;
     }
@@ -202,8 +214,9 @@ int hist_launch(pyg_ctx* ctx, const longlong2* in, int64_t n, int64_t step, int 
                 long long* mm = nullptr, const RJModel* model = nullptr);
 // Partition pass(es) of one relation into P1 (and P2 when two): *err is set
 // if a tile's bulk copy never landed, *ovf if a sampled region overflowed,
-// *frame if a tuple fell outside a packed layout's frame.  Afterwards
-// d.cur2 holds the tuples written per fine partition.
+// *frame if a tuple fell outside a packed layout's frame.  After two passes
+// d.cur2 holds the tuples written per fine partition (one pass has an exact
+// layout, whose counts are known).
 // Range mode when csplit is set: pass 1 bins by the 2^CB - 1 coarse
 // splitters, pass 2 by the fine splitters (F - 1, ascending; coarse
 // splitter i = fine splitter (i + 1) * 2^(FB - CB) - 1).
@@ -211,11 +224,18 @@ int run_passes(pyg_ctx* ctx, const longlong2* in, int64_t n, const RJLayout& L, 
                int CB, void* P1, void* P2, unsigned* err, unsigned* ovf, const long long* csplit = nullptr,
                const long long* fsplit = nullptr, unsigned* frame = nullptr, cudaEvent_t between = nullptr,
                const RJModel* model = nullptr);
-// Device bytes of a layout's pass buffers (packed buffers get 16 bytes of
-// tail so that the last tile's 16-byte-rounded copy stays inside).
+// Elements past a pass buffer's last region: the runs of bins that outgrow
+// their sampled region go there (at most one tile at a time per CTA; nothing
+// reads them), and a last tile's copy of packed words, rounded up to 16
+// bytes, stays inside the buffer.
+constexpr int RJ_DUMP = 8192;
+static_assert(RJ_DUMP >= RJ_TILE_U && RJ_DUMP >= RJ_TILE_P && RJ_DUMP >= RJ_TILE_PM && RJ_DUMP >= RJ_TILE_8 &&
+                  RJ_DUMP >= RJ_TILE_8M,
+              "a run is at most a tile");
+// Device bytes of a layout's pass buffer of `words` elements.
 inline size_t pass_bytes(const RJLayout& L, unsigned long long words)
 {
-    return (size_t)words * elem_bytes(L) + (L.packed ? 16 : 0);
+    return ((size_t)words + RJ_DUMP) * elem_bytes(L);
 }
 // Histogram of range bins (see run_passes) of in[0], in[step], ...
 int hist_launch_range(pyg_ctx* ctx, const longlong2* in, int64_t n, int64_t step, int CB, int sub,
