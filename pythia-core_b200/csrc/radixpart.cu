@@ -909,7 +909,10 @@ int rp_partition_sides(pyg_ctx* ctx, RPSide* sd, int ns, int FB, bool two, unsig
     const int F = 1 << FB;
     const size_t side = RJSideDev::words(F, 1 << coarse_bits(false));
     const size_t per = side + F + 4;  // metadata, histogram, {kmin, kmax, pmin, pmax}
-    if (ns < 1 || ns > 2 || (size_t)ns * (F + 4) * 8 > kPinnedStageBytes) {
+    // Host words per relation: the histogram and the ranges, or the cursors
+    // that hold a sampled relation's counts.
+    const size_t hper = std::max<size_t>(F, two ? 0 : (size_t)F * RJ_CURSOR_STRIDE) + 4;
+    if (ns < 1 || ns > 2 || (size_t)ns * hper * 8 > kPinnedStageBytes) {
         set_error("partition: %d relations of 2^%d partitions exceed the staging area", ns, FB);
         return PYG_ERR_ARG;
     }
@@ -924,7 +927,7 @@ int rp_partition_sides(pyg_ctx* ctx, RPSide* sd, int ns, int FB, bool two, unsig
     int rc = PYG_OK;
     for (int s = 0; s < ns; ++s) sd[s].P1 = sd[s].P2 = nullptr;
     auto hist_at = [&](int s) { return meta + (size_t)s * per + side; };
-    auto hh_at = [&](int s) { return hh + (size_t)s * (F + 4); };
+    auto hh_at = [&](int s) { return hh + (size_t)s * hper; };
     auto hist_of = [&](int s, int64_t st) {
         if (sd[s].csplit) {
             const int cb = coarse_bits(false);
@@ -969,8 +972,8 @@ int rp_partition_sides(pyg_ctx* ctx, RPSide* sd, int ns, int FB, bool two, unsig
         PYG_CUDA(cudaMemsetAsync(flags, 0, (size_t)16 * ns, ctx->stream));
         int64_t step[2] = {1, 1};
         for (int s = 0; s < ns && !rc; ++s) {
-            sample[s] = sd[s].allow_sample && two && sd[s].n >= ((int64_t)1 << 25);
-            step[s] = sample[s] ? std::max<int64_t>(1, sd[s].n >> RJ_SAMPLE_LOG2) : 1;
+            sample[s] = sd[s].allow_sample && sd[s].n >= ((int64_t)1 << 25);
+            step[s] = sample[s] ? std::max<int64_t>(1, sd[s].n >> rj_sample_log2(FB)) : 1;
             if ((rc = hist_of(s, step[s]))) break;
             sd[s].hist_tuples = (sd[s].n + step[s] - 1) / step[s];
         }
@@ -997,7 +1000,9 @@ int rp_partition_sides(pyg_ctx* ctx, RPSide* sd, int ns, int FB, bool two, unsig
         PYG_CUDA(cudaMemcpyAsync(hflags, flags, (size_t)16 * ns, cudaMemcpyDeviceToHost, ctx->stream));
         for (int s = 0; s < ns; ++s)
             if (sd[s].L.sampled)
-                PYG_CUDA(cudaMemcpyAsync(hh_at(s), d[s].cur2, (size_t)F * 8, cudaMemcpyDeviceToHost, ctx->stream));
+                PYG_CUDA(cudaMemcpyAsync(hh_at(s), two ? d[s].cur2 : d[s].cur1,
+                                         (size_t)F * 8 * (two ? 1 : RJ_CURSOR_STRIDE), cudaMemcpyDeviceToHost,
+                                         ctx->stream));
         PYG_CUDA(cudaStreamSynchronize(ctx->stream));
         for (int s = 0; s < ns && !rc; ++s) {
             if (hflags[4 * s]) {
@@ -1005,7 +1010,10 @@ int rp_partition_sides(pyg_ctx* ctx, RPSide* sd, int ns, int FB, bool two, unsig
                 rc = PYG_ERR_TIMEOUT;
                 break;
             }
-            if (sd[s].L.sampled) sd[s].L.count.assign(hh_at(s), hh_at(s) + F);
+            if (sd[s].L.sampled) {
+                sd[s].L.count.resize(F);
+                for (int f = 0; f < F; ++f) sd[s].L.count[f] = hh_at(s)[(size_t)f * (two ? 1 : RJ_CURSOR_STRIDE)];
+            }
             if (!hflags[4 * s + 1] && !hflags[4 * s + 2]) continue;
             // A sampled region overflowed, or a tuple fell outside a frame
             // taken from the sample: redo this relation from an exact

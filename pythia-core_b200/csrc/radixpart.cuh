@@ -58,13 +58,12 @@ constexpr int RJ_SPLIT_MAX = 256;        // range mode: splitters per pass segme
 // 2^15 32-bit counters in shared memory.
 constexpr int RJ_MAX_FINE_BITS = 16;   // hash mode (histograms run in halves above 2^15 bins)
 constexpr int RJ_MAX_RANGE_BITS = 15;  // range mode (one 2^15-counter histogram)
-#ifndef PYG_RJ_SAMPLE_LOG2
-#define PYG_RJ_SAMPLE_LOG2 22
-#endif
-// Sampled layouts count every (n >> RJ_SAMPLE_LOG2)-th tuple (2^22 samples:
-// at most 0.2 ms for two relations; regions get more slack than with a
-// larger sample, which costs device memory, not traffic).
-constexpr int RJ_SAMPLE_LOG2 = PYG_RJ_SAMPLE_LOG2;
+// Sampled layouts count every (n >> rj_sample_log2)-th tuple: about 2^9
+// samples per partition, at most 2^22 (0.1 ms per relation; a sample costs a
+// 32-byte sector, 78 us for 2^22 of 2^27 tuples against 12 us for 2^17).
+// Fewer samples give regions more slack, which costs device memory, not
+// traffic.
+inline int rj_sample_log2(int FB) { return FB < 8 ? 17 : (FB > 13 ? 22 : FB + 9); }
 
 // Partition bins computed by a learned CDF model instead of a search
 // (range partitioning without splitters in the passes).  For a model with
@@ -215,8 +214,8 @@ int hist_launch(pyg_ctx* ctx, const longlong2* in, int64_t n, int64_t step, int 
 // Partition pass(es) of one relation into P1 (and P2 when two): *err is set
 // if a tile's bulk copy never landed, *ovf if a sampled region overflowed,
 // *frame if a tuple fell outside a packed layout's frame.  After two passes
-// d.cur2 holds the tuples written per fine partition (one pass has an exact
-// layout, whose counts are known).
+// d.cur2 holds the tuples written per fine partition; after one, d.cur1 at
+// RJ_CURSOR_STRIDE words each.
 // Range mode when csplit is set: pass 1 bins by the 2^CB - 1 coarse
 // splitters, pass 2 by the fine splitters (F - 1, ascending; coarse
 // splitter i = fine splitter (i + 1) * 2^(FB - CB) - 1).
