@@ -1,7 +1,7 @@
 // MPSM sort-merge join on one B200.
 //
-// Pipeline (both sides carried as 16-byte items {int64 key, int64 val},
-// val = the projected column or the input row number):
+// Aggregate sink (both sides carried as 16-byte items {int64 key, int64
+// val}, val = the projected column):
 //   1. splitters: equal-width over [min, max] (the reference's
 //      ExactRangeValueHasher), quantiles of a probe-key sample, or the
 //      learned CDF model trained on that sample;
@@ -12,11 +12,13 @@
 //      that split each merge across CTAs in 2048-item output tiles;
 //   4. merge join: CTAs take (partition, probe chunk) work items; each
 //      thread merges a run of sorted probe items against the partition's
-//      sorted build run (binary search + forward scan) and either
-//      accumulates count / sums (build sums from a prefix sum over the
-//      sorted build vals) or writes the joined rows.
-// A partition's build and probe items are sorted by (key, val), so the
-// materialised output order is deterministic: key, probe row, build row.
+//      sorted build run (binary search + forward scan) and accumulates count
+//      and sums (build sums from a prefix sum over the sorted build vals).
+// 16-byte (int64, int64) device tuples take mpsm16.cu instead.
+//
+// Materialising sink: both sides sorted as a whole by key, stable (so in row
+// order within a key), and merged: rows come out ordered by key, probe row,
+// build row.
 #include <math.h>
 #include <string.h>
 
@@ -25,6 +27,7 @@
 
 #include "../../include/pyg_learned.h"
 #include "../../include/pyg_mpsm.h"
+#include "lookback.cuh"
 #include "mpsm16.cuh"
 #include "partition.cuh"
 #include "primitives.cuh"
@@ -161,17 +164,6 @@ struct JoinArgs {
     const unsigned char* spar;     // per partition: 1 if the sorted probe run is in S1
     const JoinWork* work;
     int nwork;
-    // materialise
-    int mode;                      // 0 aggregate, 1 count matches, 2 write rows
-    unsigned long long* counts;    // per probe item match count / output offset
-    const uint8_t* rbase;          // original relations (row gather)
-    const uint8_t* sbase;
-    int32_t rtb, stb;
-    int nproj;
-    int32_t pside[PYG_MAX_COLS], poff[PYG_MAX_COLS], ptype[PYG_MAX_COLS], ooff[PYG_MAX_COLS];
-    int32_t out_tb;
-    uint8_t* out;
-    int64_t out_cap;
     unsigned long long* acc;       // count, build sum, probe sum
 };
 
@@ -207,36 +199,261 @@ __global__ void __launch_bounds__(MP_JOIN_THREADS) mp_join_kernel(JoinArgs a)
                 have = true;
             }
             uint64_t c = (uint64_t)(hi - lo);
-            if (a.mode == 0) {
-                cnt += c;
-                bsum += a.rpre[hi] - a.rpre[lo];
-                psum += c * (uint64_t)s.y;
-            } else if (a.mode == 1) {
-                a.counts[i] = c;
-            } else if (c) {
-                int64_t pos = (int64_t)a.counts[i];
-                const uint8_t* st = a.sbase + (int64_t)s.y * a.stb;
-                for (int64_t r = lo; r < hi; ++r, ++pos) {
-                    if (pos >= a.out_cap) break;
-                    const uint8_t* rt = a.rbase + (int64_t)a.R[r].y * a.rtb;
-                    uint8_t* dst = a.out + pos * (int64_t)a.out_tb;
-                    for (int p = 0; p < a.nproj; ++p) {
-                        store_col(dst, a.ooff[p], a.ptype[p],
-                                  (uint64_t)load_col(a.pside[p] ? st : rt, a.poff[p], a.ptype[p]));
-                    }
-                }
-            }
+            cnt += c;
+            bsum += a.rpre[hi] - a.rpre[lo];
+            psum += c * (uint64_t)s.y;
         }
     }
-    if (a.mode == 0) {
-        cnt = warp_sum_u64(cnt);
-        bsum = warp_sum_u64(bsum);
-        psum = warp_sum_u64(psum);
-        if ((threadIdx.x & 31) == 0 && (cnt | bsum | psum)) {
-            atomicAdd(&a.acc[0], (unsigned long long)cnt);
-            atomicAdd(&a.acc[1], (unsigned long long)bsum);
-            atomicAdd(&a.acc[2], (unsigned long long)psum);
+    cnt = warp_sum_u64(cnt);
+    bsum = warp_sum_u64(bsum);
+    psum = warp_sum_u64(psum);
+    if ((threadIdx.x & 31) == 0 && (cnt | bsum | psum)) {
+        atomicAdd(&a.acc[0], (unsigned long long)cnt);
+        atomicAdd(&a.acc[1], (unsigned long long)bsum);
+        atomicAdd(&a.acc[2], (unsigned long long)psum);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Materialising sink.  Both relations' (key, value) items are sorted by key
+// with the stable radix sort, so the items of one key are in row order; then
+// one kernel walks the sorted probe items in tiles: it finds each item's run
+// of build items, learns from its predecessors how many rows come before
+// the tile (look-back) and writes the tile's rows.  The value is the one
+// projected column of the side besides the key, else the row number, whose
+// columns are gathered.
+//
+// Bound: the sorts (32 bytes per item and key byte), then the chain of a
+// tile (ticket, range search, look-back).  1 M x 6 M rows, keys of 20 bits:
+// 545 us, 128 us of them this kernel (173 us with 2048-item tiles, two CTAs
+// per SM), against 2792 us with range splitters, bitonic tiles, merge rounds,
+// a counting and a writing join by one thread per 32 probe items and row
+// gathers.
+
+constexpr int MM_THREADS = 256;
+constexpr int MM_PER = 4;
+constexpr int MM_TILE = MM_THREADS * MM_PER;  // probe items per tile
+constexpr int MM_RKEYS = 1024;                // build keys of a tile held in shared memory
+
+struct MatArgs {
+    const longlong2* R;   // sorted items
+    int64_t nR;
+    const longlong2* S;
+    int64_t nS;
+    unsigned* ticket;     // zeroed, with status
+    unsigned long long* status;
+    unsigned* err;
+    unsigned long long* total;
+    const uint8_t* rbase;  // original relations (row gather)
+    const uint8_t* sbase;
+    int32_t rtb, stb;
+    int rows16;            // output tuples are {build value, probe value}, 16-byte aligned
+    int nproj;
+    int32_t pside[PYG_MAX_COLS];  // 0 build, 1 probe
+    int32_t psrc[PYG_MAX_COLS];   // 0 the item's key, 1 its value, 2 column of its row
+    int32_t poff[PYG_MAX_COLS], ptype[PYG_MAX_COLS], ooff[PYG_MAX_COLS];
+    int32_t out_tb;
+    uint8_t* out;
+    int64_t out_cap;
+};
+
+__device__ __forceinline__ void mm_write(const MatArgs& a, int64_t pos, const longlong2& r, const longlong2& s)
+{
+    if (pos >= a.out_cap) return;
+    if (a.rows16) {
+        __stcs(reinterpret_cast<longlong2*>(a.out) + pos, make_longlong2(r.y, s.y));
+        return;
+    }
+    uint8_t* dst = a.out + pos * (int64_t)a.out_tb;
+    for (int p = 0; p < a.nproj; ++p) {
+        const longlong2& it = a.pside[p] ? s : r;
+        uint64_t v;
+        if (a.psrc[p] == 0) v = (uint64_t)it.x;
+        else if (a.psrc[p] == 1) v = (uint64_t)it.y;
+        else
+            v = (uint64_t)load_col((a.pside[p] ? a.sbase : a.rbase) + it.y * (int64_t)(a.pside[p] ? a.stb : a.rtb),
+                                   a.poff[p], a.ptype[p]);
+        store_col(dst, a.ooff[p], a.ptype[p], v);
+    }
+}
+
+__global__ void __launch_bounds__(MM_THREADS) mm_join_kernel(MatArgs a)
+{
+    __shared__ longlong2 ss[MM_TILE];
+    extern __shared__ __align__(16) unsigned char mm_smem[];
+    long long* rk = reinterpret_cast<long long*>(mm_smem);                          // MM_RKEYS
+    unsigned long long* off = reinterpret_cast<unsigned long long*>(rk + MM_RKEYS);  // MM_TILE: matches, then offsets
+    unsigned long long* first = off + MM_TILE;                                       // MM_TILE: first build item
+    __shared__ unsigned ticket;
+    __shared__ int64_t r0s, r1s;
+    __shared__ unsigned long long warp_tot[MM_THREADS / 32], base_s, total_s;
+    __shared__ int ok, many;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    if (tid == 0) {
+        ticket = atomicAdd(a.ticket, 1u);
+        ok = 1;
+        many = 0;
+    }
+    __syncthreads();
+    const int64_t tile = ticket, s0 = tile * MM_TILE;
+    const int n = a.nS - s0 < MM_TILE ? (int)(a.nS - s0) : MM_TILE;
+    for (int i = tid; i < n; i += MM_THREADS) ss[i] = a.S[s0 + i];
+    // The build items of the tile's key range: [r0, r1).
+    if (w < 2) {
+        // Warp 0: the first key >= the tile's first; warp 1: the first key >
+        // its last.  32 probes per step.
+        const long long key = a.S[w == 0 ? s0 : s0 + n - 1].x;
+        int64_t lo = 0, hi = a.nR;
+        while (lo < hi) {
+            const int64_t step = (hi - lo + 32) / 33;
+            const int64_t at = lo + (lane + 1) * step - 1;
+            bool before = false;
+            if (at < hi) {
+                const long long k = a.R[at].x;
+                before = w == 0 ? k < key : k <= key;
+            }
+            const int cnt = __popc(__ballot_sync(0xffffffffu, before));
+            const int64_t next = lo + (cnt + 1) * step - 1;  // the first probe past the answer, if there is one
+            lo += cnt * step;
+            if (cnt < 32 && next < hi) hi = next;
         }
+        if (lane == 0) (w == 0 ? r0s : r1s) = lo;
+    }
+    __syncthreads();
+    const int64_t r0 = r0s, r1 = r1s;
+    const bool held = r1 - r0 <= MM_RKEYS;
+    if (held) {
+        for (int i = tid; i < (int)(r1 - r0); i += MM_THREADS) rk[i] = a.R[r0 + i].x;
+        __syncthreads();
+    }
+    // Each item's run of build items: first index and length.
+    int64_t lo[MM_PER];
+    unsigned long long c[MM_PER];
+    bool dup = false;
+#pragma unroll
+    for (int j = 0; j < MM_PER; ++j) {
+        const int i = j * MM_THREADS + tid;
+        lo[j] = r0;
+        c[j] = 0;
+        if (i < n) {
+            const long long key = ss[i].x;
+            if (held) {
+                const int m = (int)(r1 - r0);
+                int l = 0, len = m;
+                while (len > 0) {
+                    const int half = len >> 1;
+                    if (rk[l + half] < key) {
+                        l += half + 1;
+                        len -= half + 1;
+                    } else {
+                        len = half;
+                    }
+                }
+                int e = l;
+                if (e < m && rk[e] == key) {
+                    ++e;
+                    if (e < m && rk[e] == key) {  // repeated build key: upper bound
+                        len = m - e;
+                        while (len > 0) {
+                            const int half = len >> 1;
+                            if (rk[e + half] <= key) {
+                                e += half + 1;
+                                len -= half + 1;
+                            } else {
+                                len = half;
+                            }
+                        }
+                    }
+                }
+                lo[j] = r0 + l;
+                c[j] = (unsigned long long)(e - l);
+            } else {
+                lo[j] = lower_bound_key(a.R, r0, r1, key);
+                int64_t e = lo[j];
+                if (e < r1 && a.R[e].x == key) {
+                    ++e;
+                    if (e < r1 && a.R[e].x == key) {
+                        int64_t hi = r1;
+                        while (e < hi) {
+                            const int64_t mid = e + ((hi - e) >> 1);
+                            if (a.R[mid].x <= key) e = mid + 1;
+                            else hi = mid;
+                        }
+                    }
+                }
+                c[j] = (unsigned long long)(e - lo[j]);
+            }
+            dup |= c[j] > 1;
+        }
+        off[i] = c[j];
+        first[i] = (unsigned long long)lo[j];
+    }
+    if (__any_sync(0xffffffffu, dup) && lane == 0) many = 1;
+    __syncthreads();
+    // Exclusive prefix of the match counts in item order.
+    unsigned long long v[MM_PER], sum = 0;
+#pragma unroll
+    for (int j = 0; j < MM_PER; ++j) {
+        v[j] = off[tid * MM_PER + j];
+        sum += v[j];
+    }
+    unsigned long long incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long x = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += x;
+    }
+    if (lane == 31) warp_tot[w] = incl;
+    __syncthreads();
+    unsigned long long run = incl - sum, all = 0;
+    for (int q = 0; q < MM_THREADS / 32; ++q) {
+        if (q < w) run += warp_tot[q];
+        all += warp_tot[q];
+    }
+#pragma unroll
+    for (int j = 0; j < MM_PER; ++j) {
+        off[tid * MM_PER + j] = run;
+        run += v[j];
+    }
+    // Rows before this tile.
+    if (w == 0) {
+        unsigned long long before = 0;
+        const bool found = lb_prefix(a.status, tile, all, a.err, before);
+        if (lane == 0) {
+            if (!found) ok = 0;
+            base_s = before;
+            total_s = all;
+            if (s0 + n == a.nS) *a.total = before + all;
+        }
+    }
+    __syncthreads();
+    if (!ok) return;
+    const int64_t base = (int64_t)base_s;
+    if (base >= a.out_cap) return;
+    if (!many) {
+        // At most one row per item: consecutive items write consecutive rows.
+#pragma unroll
+        for (int j = 0; j < MM_PER; ++j) {
+            const int i = j * MM_THREADS + tid;
+            if (c[j]) mm_write(a, base + (int64_t)off[i], a.R[lo[j]], ss[i]);
+        }
+        return;
+    }
+    // Rows of items with many matches are spread over the CTA: row q of the
+    // tile belongs to the last item whose offset is at most q.
+    const unsigned long long total = total_s;
+    for (unsigned long long q = tid; q < total && base + (int64_t)q < a.out_cap; q += MM_THREADS) {
+        int l = 0, len = n;
+        while (len > 1) {
+            const int half = len >> 1;
+            if (off[l + half] <= q) {
+                l += half;
+                len -= half;
+            } else {
+                len = half;
+            }
+        }
+        mm_write(a, base + (int64_t)q, a.R[first[l] + (q - off[l])], ss[l]);
     }
 }
 
@@ -370,6 +587,98 @@ struct Splits {
     std::vector<int64_t> spl;  // F - 1 splitters
 };
 
+// The materialising sink on staged relations (arguments checked).
+static int mpsm_materialize(pyg_ctx* ctx, const pyg_rel* build, const pyg_rel& R, int32_t bkey, const pyg_rel* probe,
+                            const pyg_rel& S, int32_t pkey, const pyg_proj* proj, int32_t nproj, void* out,
+                            int64_t out_cap, int64_t* out_count)
+{
+    const pyg_rel* rel[2] = {build, probe};
+    const pyg_rel* dev[2] = {&R, &S};
+    const int key[2] = {bkey, pkey};
+    const int64_t n[2] = {build->ntuples, probe->ntuples};
+    *out_count = 0;
+    if (n[0] == 0 || n[1] == 0) return PYG_OK;
+    Mpsm M{ctx, {}};
+    int rc;
+    // The value of a side's items: its only projected column besides the
+    // key, or the row number when there are more.
+    int vcol[2] = {-1, -1};
+    bool rows[2] = {false, false};
+    for (int p = 0; p < nproj; ++p) {
+        const int s = proj[p].side ? 1 : 0;
+        if (proj[p].col == key[s]) continue;
+        if (vcol[s] >= 0 && vcol[s] != proj[p].col) rows[s] = true;
+        vcol[s] = proj[p].col;
+    }
+    const ulonglong2* items[2];
+    ulonglong2* sorted[2];
+    for (int s = 0; s < 2; ++s) {
+        const pyg_rel* r = rel[s];
+        const int v = vcol[s];
+        // 16-byte tuples of an int64 key and the value are items already.
+        const bool direct = !rows[s] && r->tuple_bytes == 16 && r->col_offset[key[s]] == 0 &&
+                            r->col_type[key[s]] == PYG_INT64 && (uintptr_t)dev[s]->base % 16 == 0 &&
+                            (v < 0 || (r->col_offset[v] == 8 && r->col_type[v] == PYG_INT64));
+        if ((rc = M.alloc((void**)&sorted[s], (size_t)n[s] * 16))) return rc;
+        if (direct) {
+            items[s] = (const ulonglong2*)dev[s]->base;
+            continue;
+        }
+        longlong2* it;
+        if ((rc = M.alloc((void**)&it, (size_t)n[s] * 16))) return rc;
+        mp_extract_kernel<<<grid_for(ctx, n[s], 256, 4, 8), 256, 0, ctx->stream>>>(
+            (const uint8_t*)dev[s]->base, n[s], r->tuple_bytes, r->col_offset[key[s]], r->col_type[key[s]],
+            v >= 0 ? r->col_offset[v] : -1, v >= 0 ? r->col_type[v] : PYG_INT64, rows[s] ? 1 : 0, it);
+        PYG_LAUNCHED(ctx);
+        items[s] = (const ulonglong2*)it;
+    }
+    if ((rc = radix_sort16_two(ctx, items, sorted, n))) return rc;
+    MatArgs a;
+    memset(&a, 0, sizeof(a));
+    const int64_t tiles = (n[1] + MM_TILE - 1) / MM_TILE;
+    unsigned long long* status;
+    if ((rc = M.alloc((void**)&status, (size_t)(tiles + 1) * 8))) return rc;
+    PYG_CUDA(cudaMemsetAsync(status, 0, (size_t)(tiles + 1) * 8, ctx->stream));
+    a.R = (const longlong2*)sorted[0];
+    a.nR = n[0];
+    a.S = (const longlong2*)sorted[1];
+    a.nS = n[1];
+    a.ticket = (unsigned*)(status + tiles);
+    a.status = status;
+    a.err = (unsigned*)(ctx->dcounters + SORT_ERR_WORD);
+    a.total = ctx->dcounters + 112;
+    a.rbase = (const uint8_t*)R.base;
+    a.sbase = (const uint8_t*)S.base;
+    a.rtb = build->tuple_bytes;
+    a.stb = probe->tuple_bytes;
+    a.nproj = nproj;
+    for (int p = 0; p < nproj; ++p) {
+        const int s = proj[p].side ? 1 : 0;
+        a.pside[p] = s;
+        a.psrc[p] = proj[p].col == key[s] ? 0 : (rows[s] ? 2 : 1);
+        a.poff[p] = rel[s]->col_offset[proj[p].col];
+        a.ptype[p] = rel[s]->col_type[proj[p].col];
+        a.ooff[p] = a.out_tb;
+        a.out_tb += a.ptype[p] == PYG_INT32 ? 4 : 8;
+    }
+    a.rows16 = nproj == 2 && a.pside[0] == 0 && a.pside[1] == 1 && a.psrc[0] == 1 && a.psrc[1] == 1 &&
+               a.ptype[0] == PYG_INT64 && a.ptype[1] == PYG_INT64 && (uintptr_t)out % 16 == 0;
+    a.out = (uint8_t*)out;
+    a.out_cap = out_cap;
+    const int smem = MM_RKEYS * 8 + MM_TILE * 16;
+    PYG_CUDA(cudaFuncSetAttribute(mm_join_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    mm_join_kernel<<<(unsigned)tiles, MM_THREADS, smem, ctx->stream>>>(a);
+    PYG_LAUNCHED(ctx);
+    unsigned long long* h = (unsigned long long*)ctx->pinned + 256;
+    PYG_CUDA(cudaMemcpyAsync(h, a.total, 8, cudaMemcpyDeviceToHost, ctx->stream));
+    PYG_CUDA(cudaMemcpyAsync((unsigned long long*)ctx->pinned + SORT_ERR_PINNED, ctx->dcounters + SORT_ERR_WORD, 8,
+                             cudaMemcpyDeviceToHost, ctx->stream));
+    PYG_CUDA(cudaStreamSynchronize(ctx->stream));
+    if ((rc = sort_status(ctx))) return rc;
+    *out_count = (int64_t)h[0];
+    return PYG_OK;
+}
+
 static int mpsm_run(pyg_ctx* ctx, const pyg_rel* build, int32_t bkey, const pyg_rel* probe, int32_t pkey,
                     const pyg_proj* proj, int32_t nproj, const pyg_mpsm_opts* o, bool materialize, void* out,
                     int64_t out_cap, int64_t* out_count, pyg_join_result* res, pyg_mpsm_stats* stats)
@@ -413,6 +722,25 @@ static int mpsm_run(pyg_ctx* ctx, const pyg_rel* build, int32_t bkey, const pyg_
     }
     const int F = o->fanout;
     const int64_t nR = build->ntuples, nS = probe->ntuples;
+    if (materialize) {
+        // The order by key leaves nothing to the range splitters; a learned
+        // model that could not be trained is refused all the same.
+        if (o->splitter_kind == PYG_MPSM_SPLIT_LEARNED && F > 1 && nS > 0 && nR + nS >= 2 && o->cdf_leaves > (1 << 20)) {
+            set_error("mpsm: 1..2^20 leaves");
+            return PYG_ERR_ARG;
+        }
+        DevRel Rd, Sd;
+        if (!(rc = Rd.stage(ctx, build)) && !(rc = Sd.stage(ctx, probe)))
+            rc = mpsm_materialize(ctx, build, Rd.rel, bkey, probe, Sd.rel, pkey, proj, nproj, out, out_cap, out_count);
+        Rd.release(ctx);
+        Sd.release(ctx);
+        if (rc) return rc;
+        if (*out_count > out_cap) {
+            set_error("mpsm: %lld joined rows exceed capacity %lld", (long long)*out_count, (long long)out_cap);
+            return PYG_ERR_CAPACITY;
+        }
+        return PYG_OK;
+    }
     Mpsm M{ctx, {}};
     cudaEvent_t ev[5];
     for (auto& e : ev) cudaEventCreate(&e);
@@ -433,7 +761,7 @@ static int mpsm_run(pyg_ctx* ctx, const pyg_rel* build, int32_t bkey, const pyg_
     // 16-byte items {key, val}.
     auto items_of = [&](const pyg_rel* r, const pyg_rel& dev, int key, int col, int64_t n,
                         longlong2** items) -> int {
-        bool direct = !materialize && r->tuple_bytes == 16 && r->col_offset[key] == 0 &&
+        bool direct = r->tuple_bytes == 16 && r->col_offset[key] == 0 &&
                       r->col_type[key] == PYG_INT64 && (col < 0 || (r->col_offset[col] == 8 && r->col_type[col] == PYG_INT64)) &&
                       col >= 0 && (uintptr_t)dev.base % 16 == 0;
         if (direct) {
@@ -445,7 +773,7 @@ static int mpsm_run(pyg_ctx* ctx, const pyg_rel* build, int32_t bkey, const pyg_
         if (n > 0) {
             mp_extract_kernel<<<grid_for(ctx, n, 256, 4, 8), 256, 0, ctx->stream>>>(
                 (const uint8_t*)dev.base, n, r->tuple_bytes, r->col_offset[key], r->col_type[key],
-                col >= 0 ? r->col_offset[col] : -1, col >= 0 ? r->col_type[col] : PYG_INT64, materialize ? 1 : 0,
+                col >= 0 ? r->col_offset[col] : -1, col >= 0 ? r->col_type[col] : PYG_INT64, 0,
                 *items);
             PYG_LAUNCHED(ctx);
         }
@@ -463,7 +791,7 @@ static int mpsm_run(pyg_ctx* ctx, const pyg_rel* build, int32_t bkey, const pyg_
                (col < 0 || (col == 1 && r->col_offset[1] == 8 && r->col_type[1] == PYG_INT64)) &&
                (uintptr_t)r->base % 16 == 0;
     };
-    const bool fast = !materialize && is16(build, bkey, bcol) && is16(probe, pkey, pcol) && nR > 0 && nS > 0;
+    const bool fast = is16(build, bkey, bcol) && is16(probe, pkey, pcol) && nR > 0 && nS > 0;
     const int FBf = fast ? mpsm16_fine_bits(nR, nS) : 0;
     const int Fs = fast ? (1 << FBf) : F;
 
@@ -619,11 +947,9 @@ static int mpsm_run(pyg_ctx* ctx, const pyg_rel* build, int32_t bkey, const pyg_
     cudaEventRecord(ev[2], ctx->stream);
     PYG_CUDA(cudaStreamSynchronize(ctx->stream));
 
-    // A partition whose splitter range holds one key value needs no sort
-    // for the aggregate sink (the materialising sink still orders rows).
+    // A partition whose splitter range holds one key value needs no sort.
     std::vector<unsigned char> single(F, 0);
-    if (!materialize)
-        for (int p = 1; p + 1 < F; ++p) single[p] = spl[p] - spl[p - 1] == 1 ? 1 : 0;
+    for (int p = 1; p + 1 < F; ++p) single[p] = spl[p] - spl[p - 1] == 1 ? 1 : 0;
 
     // ---- 3. sort partitions
     std::vector<unsigned char> rpar, spar;
@@ -683,61 +1009,19 @@ static int mpsm_run(pyg_ctx* ctx, const pyg_rel* build, int32_t bkey, const pyg_
     ja.acc = acc;
     PYG_CUDA(cudaMemsetAsync(acc, 0, 24, ctx->stream));
     int jgrid = (int)std::min<size_t>(jw.size() > 0 ? jw.size() : 1, (size_t)ctx->sm_count * 8);
-    if (!materialize) {
-        ja.mode = 0;
-        if (!jw.empty()) {
-            mp_join_kernel<<<jgrid, MP_JOIN_THREADS, 0, ctx->stream>>>(ja);
-            PYG_LAUNCHED(ctx);
-        }
-        cudaEventRecord(ev[4], ctx->stream);
-        PYG_CUDA(cudaMemcpyAsync(h, acc, 24, cudaMemcpyDeviceToHost, ctx->stream));
-        PYG_CUDA(cudaStreamSynchronize(ctx->stream));
-        memset(res, 0, sizeof(*res));
-        res->count = (int64_t)h[0];
-        for (int p = 0; p < nproj; ++p) {
-            uint64_t v = proj[p].side ? h[2] : h[1];
-            int32_t t = (proj[p].side ? probe : build)->col_type[proj[p].col];
-            res->sums[p] = t == PYG_INT32 ? (int64_t)(int32_t)(uint32_t)v : (int64_t)v;
-        }
-    } else {
-        unsigned long long* counts;
-        if ((rc = M.alloc((void**)&counts, (size_t)(nS + 1) * 8))) return fail(rc);
-        PYG_CUDA(cudaMemsetAsync(counts, 0, (size_t)(nS + 1) * 8, ctx->stream));
-        ja.counts = counts;
-        ja.mode = 1;
-        if (!jw.empty()) {
-            mp_join_kernel<<<jgrid, MP_JOIN_THREADS, 0, ctx->stream>>>(ja);
-            PYG_LAUNCHED(ctx);
-        }
-        unsigned long long* total = ctx->dcounters + 112;
-        if ((rc = exclusive_scan_u64(ctx, counts, counts, nS + 1, total))) return fail(rc);
-        PYG_CUDA(cudaMemcpyAsync(h, total, 8, cudaMemcpyDeviceToHost, ctx->stream));
-        PYG_CUDA(cudaStreamSynchronize(ctx->stream));
-        *out_count = (int64_t)h[0];
-        ja.mode = 2;
-        ja.rbase = (const uint8_t*)Rd.rel.base;
-        ja.sbase = (const uint8_t*)Sd.rel.base;
-        ja.rtb = build->tuple_bytes;
-        ja.stb = probe->tuple_bytes;
-        ja.nproj = nproj;
-        int ob = 0;
-        for (int p = 0; p < nproj; ++p) {
-            const pyg_rel* r = proj[p].side ? probe : build;
-            ja.pside[p] = proj[p].side ? 1 : 0;
-            ja.poff[p] = r->col_offset[proj[p].col];
-            ja.ptype[p] = r->col_type[proj[p].col];
-            ja.ooff[p] = ob;
-            ob += ja.ptype[p] == PYG_INT32 ? 4 : 8;
-        }
-        ja.out_tb = ob;
-        ja.out = (uint8_t*)out;
-        ja.out_cap = out_cap;
-        if (!jw.empty() && out_cap > 0 && nproj > 0) {
-            mp_join_kernel<<<jgrid, MP_JOIN_THREADS, 0, ctx->stream>>>(ja);
-            PYG_LAUNCHED(ctx);
-        }
-        cudaEventRecord(ev[4], ctx->stream);
-        PYG_CUDA(cudaStreamSynchronize(ctx->stream));
+    if (!jw.empty()) {
+        mp_join_kernel<<<jgrid, MP_JOIN_THREADS, 0, ctx->stream>>>(ja);
+        PYG_LAUNCHED(ctx);
+    }
+    cudaEventRecord(ev[4], ctx->stream);
+    PYG_CUDA(cudaMemcpyAsync(h, acc, 24, cudaMemcpyDeviceToHost, ctx->stream));
+    PYG_CUDA(cudaStreamSynchronize(ctx->stream));
+    memset(res, 0, sizeof(*res));
+    res->count = (int64_t)h[0];
+    for (int p = 0; p < nproj; ++p) {
+        uint64_t v = proj[p].side ? h[2] : h[1];
+        int32_t t = (proj[p].side ? probe : build)->col_type[proj[p].col];
+        res->sums[p] = t == PYG_INT32 ? (int64_t)(int32_t)(uint32_t)v : (int64_t)v;
     }
     if (stats) {
         memset(stats, 0, sizeof(*stats));
@@ -753,10 +1037,6 @@ static int mpsm_run(pyg_ctx* ctx, const pyg_rel* build, int32_t bkey, const pyg_
         stats->merge_ms = t[3];
     }
     fail(0);
-    if (materialize && *out_count > out_cap) {
-        set_error("mpsm: %lld joined rows exceed capacity %lld", (long long)*out_count, (long long)out_cap);
-        return PYG_ERR_CAPACITY;
-    }
     return PYG_OK;
 }
 

@@ -18,11 +18,18 @@ int exclusive_scan_u64(pyg_ctx* ctx, const unsigned long long* in, unsigned long
 //
 // Into out (may not alias in).
 int radix_sort16_to(pyg_ctx* ctx, const ulonglong2* in, ulonglong2* out, int64_t n, int field, bool is_signed);
+// Two relations of (signed key, value) elements by the key, with one
+// synchronisation for both key ranges.
+int radix_sort16_two(pyg_ctx* ctx, const ulonglong2* const in[2], ulonglong2* const out[2], const int64_t n[2]);
 int radix_sort8_to(pyg_ctx* ctx, const uint64_t* in, uint64_t* out, int64_t n, bool is_signed);
 // Unsigned order, both buffers overwritten; *result is the one holding the
 // sorted elements.
 int radix_sort16_swap(pyg_ctx* ctx, ulonglong2* a, ulonglong2* b, int64_t n, int field, ulonglong2** result);
 int sort_status(pyg_ctx* ctx);
+// The counter word that such a wait sets (zero since the context was made)
+// and its pinned copy, which sort_status reads and clears.
+constexpr int SORT_ERR_WORD = 36;
+constexpr int SORT_ERR_PINNED = 1000;
 
 // Order-preserving map of a signed 64-bit value to an unsigned one.
 __host__ __device__ __forceinline__ uint64_t to_sortable(int64_t v)

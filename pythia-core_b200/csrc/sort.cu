@@ -2,7 +2,7 @@
 // points (reference SortOp and TupleBuffer::sort / findsmallest).
 #include <string.h>
 
-#include "bulk.cuh"
+#include "lookback.cuh"
 #include "primitives.cuh"
 
 namespace pyg {
@@ -142,18 +142,10 @@ int exclusive_scan_u64(pyg_ctx* ctx, const unsigned long long* in, unsigned long
 // 1234; 512 x 6, 2: 1243; 256 x 16, 3 and 512 x 12, 2 spill registers
 // (1311, 1283).
 //
-// A tile waits only for tiles with smaller tickets, whose CTAs are already
-// running and never wait for it, so every wait ends; the waits are bounded
-// all the same and report an error.
+// The waits of the look-back are bounded (lookback.cuh).
 
 constexpr int OS_BINS = 256;
 constexpr int OS_MAX_PASSES = 8;
-constexpr unsigned long long kOsWaitNs = 2000000000ULL;  // 2 s
-// A pass whose bounded wait gave up sets this counter word (zero since the
-// context was made); sort_status reads its pinned copy after the caller's
-// next synchronisation and clears it.
-constexpr int OS_ERR_WORD = 36;
-constexpr int OS_ERR_PINNED = 1000;
 
 // Elements: 16-byte {x, y} sorted by word FIELD, or bare 8-byte keys.
 template <typename Item, int FIELD>
@@ -303,18 +295,6 @@ __global__ void __launch_bounds__(512) os_hist_kernel(const Item* __restrict__ i
     }
 }
 
-__device__ __forceinline__ unsigned long long os_load_status(const unsigned long long* p)
-{
-    unsigned long long v;
-    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
-}
-
-__device__ __forceinline__ void os_store_status(unsigned long long* p, unsigned long long v)
-{
-    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-
 // Elements of digit `d` in the tiles before `tile`: walks the predecessors'
 // status words back to the nearest inclusive count, LOOK words in flight
 // per step.  false when the wait gave up.
@@ -327,7 +307,7 @@ __device__ bool os_look_back(const unsigned long long* status, int64_t tile, int
     for (;;) {
         unsigned long long v[LOOK];
 #pragma unroll
-        for (int q = 0; q < LOOK; ++q) v[q] = j - q >= 0 ? os_load_status(status + (j - q) * OS_BINS + d) : 0ULL;
+        for (int q = 0; q < LOOK; ++q) v[q] = j - q >= 0 ? lb_load(status + (j - q) * OS_BINS + d) : 0ULL;
         int used = 0;
         bool open = true;
 #pragma unroll
@@ -349,7 +329,7 @@ __device__ bool os_look_back(const unsigned long long* status, int64_t tile, int
         if (used == 0) {
             const unsigned long long now = bulk_now_ns();
             if (t0 == 0) t0 = now;
-            else if (now - t0 > kOsWaitNs || *(volatile unsigned*)err) {
+            else if (now - t0 > kLookBackWaitNs || *(volatile unsigned*)err) {
                 atomicOr(err, 1u);
                 return false;
             }
@@ -428,7 +408,7 @@ __global__ void __launch_bounds__(OsShape<Item>::THREADS, OsShape<Item>::MINB)
     if (tid < OS_BINS) {
         for (int v = 0; v < WARPS; ++v) c += wcnt[v][tid];
         const unsigned real = tid == OS_BINS - 1 ? c - (unsigned)(TILE - count) : c;
-        os_store_status(st + tid, ((unsigned long long)real << 8) | (tile == 0 ? agg_tag + 1 : agg_tag));
+        lb_store(st + tid, ((unsigned long long)real << 8) | (tile == 0 ? agg_tag + 1 : agg_tag));
         incl = c;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -461,7 +441,7 @@ __global__ void __launch_bounds__(OsShape<Item>::THREADS, OsShape<Item>::MINB)
         if (tile > 0) {
             if (!os_look_back(status, tile, tid, agg_tag, err, before)) ok = 0;
             const unsigned real = tid == OS_BINS - 1 ? c - (unsigned)(TILE - count) : c;
-            os_store_status(st + tid, ((before + real) << 8) | (agg_tag + 1));
+            lb_store(st + tid, ((before + real) << 8) | (agg_tag + 1));
         }
         gbase[tid] = sc->hist[pass][tid] + before - start;
     }
@@ -532,20 +512,38 @@ struct OsPlan {
     int passes = 0;
 };
 
+// Launches the range reading of n > 0 elements into counter words 32 + 2
+// slot; os_plan_read turns the words into a plan after a synchronisation.
 template <typename Item, int FIELD>
-static int os_plan(pyg_ctx* ctx, const Item* in, int64_t n, bool is_signed, OsPlan* plan)
+static int os_plan_launch(pyg_ctx* ctx, const Item* in, int64_t n, bool is_signed, int slot)
 {
     const uint64_t flip = is_signed ? 0x8000000000000000ULL : 0ULL;
-    unsigned long long* words = ctx->dcounters + 32;
+    unsigned long long* words = ctx->dcounters + 32 + 2 * slot;
     PYG_CUDA(cudaMemsetAsync(words, 0xFF, 16, ctx->stream));
     os_range_kernel<Item, FIELD><<<grid_for(ctx, n, 512, 4, 4), 512, 0, ctx->stream>>>(in, n, flip, words);
     PYG_LAUNCHED(ctx);
-    unsigned long long* h = (unsigned long long*)ctx->pinned + 64;
-    PYG_CUDA(cudaMemcpyAsync(h, words, 16, cudaMemcpyDeviceToHost, ctx->stream));
-    PYG_CUDA(cudaStreamSynchronize(ctx->stream));
+    PYG_CUDA(cudaMemcpyAsync((unsigned long long*)ctx->pinned + 64 + 2 * slot, words, 16, cudaMemcpyDeviceToHost,
+                             ctx->stream));
+    return PYG_OK;
+}
+
+static OsPlan os_plan_read(pyg_ctx* ctx, bool is_signed, int slot)
+{
+    const unsigned long long* h = (const unsigned long long*)ctx->pinned + 64 + 2 * slot;
     const uint64_t lo = h[0], hi = ~h[1];
-    plan->base = lo ^ flip;
-    plan->passes = hi == lo ? 0 : (64 - __builtin_clzll(hi - lo) + 7) / 8;
+    OsPlan plan;
+    plan.base = lo ^ (is_signed ? 0x8000000000000000ULL : 0ULL);
+    plan.passes = hi == lo ? 0 : (64 - __builtin_clzll(hi - lo) + 7) / 8;
+    return plan;
+}
+
+template <typename Item, int FIELD>
+static int os_plan(pyg_ctx* ctx, const Item* in, int64_t n, bool is_signed, OsPlan* plan)
+{
+    int rc = os_plan_launch<Item, FIELD>(ctx, in, n, is_signed, 0);
+    if (rc) return rc;
+    PYG_CUDA(cudaStreamSynchronize(ctx->stream));
+    *plan = os_plan_read(ctx, is_signed, 0);
     return PYG_OK;
 }
 
@@ -573,11 +571,11 @@ static int os_passes(pyg_ctx* ctx, const Item* in, Item* dst0, Item* dst1, int64
         for (int p = 0; p < plan.passes; ++p) {
             Item* dst = p & 1 ? dst1 : dst0;
             kern<<<(unsigned)tiles, S::THREADS, S::SMEM, ctx->stream>>>(src, dst, n, plan.base, p, sc, status,
-                                                                  (unsigned*)(ctx->dcounters + OS_ERR_WORD));
+                                                                  (unsigned*)(ctx->dcounters + SORT_ERR_WORD));
             PYG_LAUNCHED(ctx);
             src = dst;
         }
-        PYG_CUDA(cudaMemcpyAsync((unsigned long long*)ctx->pinned + OS_ERR_PINNED, ctx->dcounters + OS_ERR_WORD, 8,
+        PYG_CUDA(cudaMemcpyAsync((unsigned long long*)ctx->pinned + SORT_ERR_PINNED, ctx->dcounters + SORT_ERR_WORD, 8,
                                  cudaMemcpyDeviceToHost, ctx->stream));
         return PYG_OK;
     };
@@ -588,10 +586,10 @@ static int os_passes(pyg_ctx* ctx, const Item* in, Item* dst0, Item* dst1, int64
 
 int sort_status(pyg_ctx* ctx)
 {
-    unsigned long long* h = (unsigned long long*)ctx->pinned + OS_ERR_PINNED;
+    unsigned long long* h = (unsigned long long*)ctx->pinned + SORT_ERR_PINNED;
     if (*h == 0) return PYG_OK;
     *h = 0;
-    PYG_CUDA(cudaMemsetAsync(ctx->dcounters + OS_ERR_WORD, 0, 8, ctx->stream));
+    PYG_CUDA(cudaMemsetAsync(ctx->dcounters + SORT_ERR_WORD, 0, 8, ctx->stream));
     set_error("sort: a bounded wait for an earlier tile gave up");
     return PYG_ERR_TIMEOUT;
 }
@@ -605,6 +603,23 @@ static int os_small(pyg_ctx* ctx, const Item* in, Item* out, int64_t n, bool is_
     return PYG_OK;
 }
 
+// The passes into out, whose last one writes it.
+template <typename Item, int FIELD>
+static int os_run_to(pyg_ctx* ctx, const Item* in, Item* out, int64_t n, const OsPlan& plan)
+{
+    if (plan.passes == 0) {  // one key value: the input order is the answer
+        PYG_CUDA(cudaMemcpyAsync(out, in, (size_t)n * sizeof(Item), cudaMemcpyDeviceToDevice, ctx->stream));
+        return PYG_OK;
+    }
+    Item* tmp = nullptr;
+    int rc;
+    if (plan.passes > 1 && (rc = dalloc(ctx, (void**)&tmp, (size_t)n * sizeof(Item)))) return rc;
+    rc = plan.passes & 1 ? os_passes<Item, FIELD>(ctx, in, out, tmp, n, plan)
+                         : os_passes<Item, FIELD>(ctx, in, tmp, out, n, plan);
+    dfree(ctx, tmp);
+    return rc;
+}
+
 template <typename Item, int FIELD>
 static int os_sort_to(pyg_ctx* ctx, const Item* in, Item* out, int64_t n, bool is_signed)
 {
@@ -612,18 +627,26 @@ static int os_sort_to(pyg_ctx* ctx, const Item* in, Item* out, int64_t n, bool i
     if (n <= OS_SMALL) return os_small<Item, FIELD>(ctx, in, out, n, is_signed);
     OsPlan plan;
     int rc = os_plan<Item, FIELD>(ctx, in, n, is_signed, &plan);
-    if (rc) return rc;
-    if (plan.passes == 0) {  // one key value: the input order is the answer
-        PYG_CUDA(cudaMemcpyAsync(out, in, (size_t)n * sizeof(Item), cudaMemcpyDeviceToDevice, ctx->stream));
-        return PYG_OK;
+    return rc ? rc : os_run_to<Item, FIELD>(ctx, in, out, n, plan);
+}
+
+int radix_sort16_two(pyg_ctx* ctx, const ulonglong2* const in[2], ulonglong2* const out[2], const int64_t n[2])
+{
+    int rc;
+    bool wait = false;
+    for (int s = 0; s < 2; ++s)
+        if (n[s] > OS_SMALL) {
+            if ((rc = os_plan_launch<ulonglong2, 0>(ctx, in[s], n[s], true, s))) return rc;
+            wait = true;
+        }
+    if (wait) PYG_CUDA(cudaStreamSynchronize(ctx->stream));
+    for (int s = 0; s < 2; ++s) {
+        if (n[s] <= 0) continue;
+        if (n[s] <= OS_SMALL) rc = os_small<ulonglong2, 0>(ctx, in[s], out[s], n[s], true);
+        else rc = os_run_to<ulonglong2, 0>(ctx, in[s], out[s], n[s], os_plan_read(ctx, true, s));
+        if (rc) return rc;
     }
-    Item* tmp = nullptr;
-    if (plan.passes > 1 && (rc = dalloc(ctx, (void**)&tmp, (size_t)n * sizeof(Item)))) return rc;
-    // The last pass writes out.
-    rc = plan.passes & 1 ? os_passes<Item, FIELD>(ctx, in, out, tmp, n, plan)
-                         : os_passes<Item, FIELD>(ctx, in, tmp, out, n, plan);
-    dfree(ctx, tmp);
-    return rc;
+    return PYG_OK;
 }
 
 int radix_sort16_to(pyg_ctx* ctx, const ulonglong2* in, ulonglong2* out, int64_t n, int field, bool is_signed)
