@@ -2,6 +2,7 @@
 #pragma once
 
 #include "pyg_internal.cuh"
+#include "radixpart.cuh"
 
 // Open-addressing table of cap slots, W 64-bit words per slot: word 0 is
 // the packed key (kEmptyKey marks a free slot), words 1..W-1 hold the
@@ -24,3 +25,19 @@ struct pyg_hashtable {
     int32_t has_dups = 0;
     int64_t entries = 0;
 };
+
+namespace pyg {
+
+// Home slot of packed key k in a table of cap slots: the radix operators'
+// hash (rj_hash), whose top bits spread a dense key range evenly, scaled by a
+// 32-bit multiply-high where 32 hash bits resolve the slots finely enough.
+// A random hash at half load gives a warp of 32 x 4 lookups a longest chain of
+// about ten dependent reads; consecutive keys here hardly meet: build of 1 M
+// keys 67 -> 19 us, materialising probe of 8 M 163 -> 88 us (against mix64).
+__device__ __forceinline__ uint64_t ht_slot(uint64_t k, uint64_t cap)
+{
+    const uint64_t h = rj_hash(k);
+    return cap <= ((uint64_t)1 << 28) ? (uint64_t)__umulhi((unsigned)(h >> 32), (unsigned)cap) : reduce_range(h, cap);
+}
+
+}  // namespace pyg
