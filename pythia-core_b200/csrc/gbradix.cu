@@ -393,9 +393,10 @@ int groupby16_fill(pyg_ctx* ctx, const void* in, int64_t n, bool pair32, int wan
                       : launch_fold(ctx, gbr_direct_kernel<GBR_PAIR>, grid, GBR_THREADS, GBR_SMEM, a);
     }
     // Partition so that each partition holds at most about GBR_PART_GROUPS
-    // keys; a large input into at least 2^GBR_PART_BITS partitions, so that
-    // most are folded and flushed once, by one CTA.
-    int FB = n >= ((int64_t)1 << 22) ? GBR_PART_BITS : 1;
+    // keys, and into at least 2^GBR_PART_BITS partitions, so that most are
+    // folded and flushed once, by one CTA (2.9 M tuples, 3817 groups: 330 us
+    // in two partitions of 23 chunks each).
+    int FB = n >= ((int64_t)1 << 17) ? GBR_PART_BITS : 1;
     while (FB < RJ_MAX_FINE_BITS && (double)expected_groups / (double)(1 << FB) > (double)GBR_PART_GROUPS) ++FB;
     const bool two = FB > RJ_MAX_LOCAL_BITS;
     const int F = 1 << FB;
@@ -413,7 +414,7 @@ int groupby16_fill(pyg_ctx* ctx, const void* in, int64_t n, bool pair32, int wan
         // Work items: whole partitions, or chunks of a large one, small
         // enough for about four items per SM.
         const unsigned long long chunk = (unsigned long long)std::max<int64_t>(
-            (int64_t)1 << 16, std::min<int64_t>(GBR_CHUNK, n / (4 * (int64_t)ctx->sm_count) + 1));
+            (int64_t)1 << 14, std::min<int64_t>(GBR_CHUNK, n / (4 * (int64_t)ctx->sm_count) + 1));
         std::vector<unsigned long long> istart;
         std::vector<unsigned> ilen;
         for (int f = 0; f < F; ++f)
