@@ -6,14 +6,15 @@
  * thread pool.  Here many PK-FK hash join + sum fragments of uneven size
  * run as one persistent kernel over a shared device work queue: per
  * fragment, table-clear items, then build items, then probe items, queued
- * shortest fragment first.  A probe item waits (with a bounded spin that
- * reports PYG_ERR_TIMEOUT instead of hanging) only for build items of its
- * own fragment that other CTAs already dequeued.  The queue reset and the
+ * shortest fragment first, in waves whose tables stay in L2 together (a
+ * wave's clear and build items before the probe items of the wave before
+ * it).  A probe item waits (with a bounded spin that reports
+ * PYG_ERR_TIMEOUT instead of hanging) only for build items of its own
+ * fragment that other CTAs already dequeued.  The queue reset and the
  * kernel are captured once in a CUDA graph and replayed per run.
  *
  * Fragments whose build side has at least `large_build` tuples are not
- * queued: their tables would not stay in L2 beside the others', and their
- * work dwarfs a call's fixed cost, so after the graph they run one by one
+ * queued: their tables would not stay in L2, so after the graph they run one by one
  * with the algorithm pyg_hashjoin_agg would pick.  Those that take the
  * direct join are enqueued back to back with no host synchronisation
  * between them (their counters stay on the device until the run's single
@@ -49,7 +50,8 @@ typedef struct pyg_tuning {
     float load_factor;           /* per-fragment table load factor           */
     int32_t chunk_tuples;        /* work-item grain in tuples                */
     int32_t large_build;         /* build tuples from which a fragment runs
-                                    as its own join (0: 2^16)             */
+                                    as its own join (0: 2^21, and those
+                                    beyond 1.3 GB of queued tables)       */
 } pyg_tuning;
 
 /* Plans n fragments (tuning NULL: the autotuner's cached choice, else

@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "../../include/pyg_batch.h"
+#include "hashtable.cuh"
 #include "pyg_internal.cuh"
 #include "radixjoin.cuh"
 
@@ -51,11 +52,21 @@ struct BatchState {
 
 constexpr int RES_WORDS = 6;  // count, sum, then empty-marker key stats: build count/sum, probe count/sum
 constexpr long long kWaitLimit = 1LL << 22;  // x ~256 ns sleeps, about one second
-// Build tuples from which a fragment runs as its own join by default.  On
-// a mix of 256 fragments with builds of 2^12..2^22 tuples, sending builds of
-// 2^16 and more to their own calls measured fastest (58.4 ms against 61.0
-// ms at 2^14 and 61.4-80.7 ms at 2^20 and above).
-constexpr int64_t kLargeBuild = (int64_t)1 << 16;
+// Build tuples from which a fragment runs as its own join by default: the
+// size from which the automatic algorithm partitions.  Below it a fragment's
+// own join would be three launches of the same work.  96 fragments with
+// builds of 2^10..2^20, 280 M tuples: 2469 us with builds of 2^16 and more as
+// their own calls, 2101 us from 2^18, 1948 us from 2^21.
+constexpr int64_t kLargeBuild = (int64_t)1 << 21;
+// By default at most this many table slots (20 bytes each) are queued, the
+// smallest fragments first; the others run as their own joins, whose table
+// is one buffer that they share.
+constexpr uint64_t kQueueSlots = (uint64_t)1 << 26;
+// The threshold when even that much memory cannot be had.
+constexpr int64_t kLargeBuildLowMem = (int64_t)1 << 16;
+// Table slots of one wave of queued fragments (16 MB; two waves are live at
+// a time, beside the probe stream, in the 126 MB L2).
+constexpr uint64_t kWaveSlots = (uint64_t)1 << 20;
 
 struct BatchDev {
     const FragDesc* frags;
@@ -145,7 +156,7 @@ __global__ void __launch_bounds__(1024) batch_kernel(BatchDev d)
 #pragma unroll
                 for (int u = 0; u < BATCH_U; ++u) {
                     const uint64_t k = (uint64_t)t[u].x;
-                    s[u] = reduce_range(mix64(k), f.cap);
+                    s[u] = ht_slot(k, f.cap);
                     pv[u] = k == kEmptyKey ? ~0ULL
                                            : (unsigned long long)atomicCAS((unsigned __int128*)&f.table[s[u]], empty,
                                                                            bslot(k, (uint64_t)t[u].y));
@@ -195,7 +206,7 @@ __global__ void __launch_bounds__(1024) batch_kernel(BatchDev d)
                 }
 #pragma unroll
                 for (int u = 0; u < BATCH_U; ++u) {
-                    s[u] = reduce_range(mix64((uint64_t)t[u].x), f.cap);
+                    s[u] = ht_slot((uint64_t)t[u].x, f.cap);
                     e[u] = f.table[s[u]];
                 }
 #pragma unroll
@@ -280,8 +291,8 @@ static std::map<std::string, pyg_tuning> g_tune_cache;
 static pyg_tuning default_tuning()
 {
     pyg_tuning t;
-    t.block_threads = 512;
-    t.blocks_per_sm = 2;
+    t.block_threads = 256;
+    t.blocks_per_sm = 4;
     t.load_factor = 0.5f;
     t.chunk_tuples = 4096;
     t.large_build = 0;
@@ -428,8 +439,6 @@ int pyg_batch_create(pyg_ctx* ctx, const pyg_fragment* frags, int32_t n, const p
         pyg_batch_free(ctx, b);
         return rc;
     }
-    // Work list: fragments in ascending size (shortest first), each as
-    // clear, build, then probe items.
     std::vector<int32_t> order(n);
     for (int i = 0; i < n; ++i) order[i] = i;
     std::stable_sort(order.begin(), order.end(), [&](int a, int c) {
@@ -452,13 +461,40 @@ int pyg_batch_create(pyg_ctx* ctx, const pyg_fragment* frags, int32_t n, const p
         f.table = arena + toff[i];
         f.extra = extra + toff[i];
         f.n_init = f.n_build = f.n_probe = 0;
-        for (uint64_t s = 0; s < f.cap; s += (uint64_t)grain * 2, ++f.n_init)
-            items.push_back({i, 0, (int64_t)s, (int64_t)std::min<uint64_t>(f.cap, s + grain * 2)});
-        for (int64_t s = 0; s < f.nb; s += grain, ++f.n_build)
-            items.push_back({i, 1, s, std::min<int64_t>(f.nb, s + grain)});
-        for (int64_t s = 0; s < f.np; s += grain, ++f.n_probe)
-            items.push_back({i, 2, s, std::min<int64_t>(f.np, s + grain)});
     }
+    // Waves of fragments whose tables stay in L2 together: a wave's clear
+    // items, its build items, then the probe items of the wave before, so
+    // that the tables a probe item waits for were built a wave earlier.
+    // (Clear, build and probe of one fragment after another kept most CTAs
+    // waiting: 57 fragments of 16 M tuples took 1093 us.)
+    auto probes = [&](size_t w0, size_t w1) {
+        for (size_t q = w0; q < w1; ++q) {
+            FragDesc& f = fd[order[q]];
+            for (int64_t s = 0; s < f.np; s += grain, ++f.n_probe)
+                items.push_back({order[q], 2, s, std::min<int64_t>(f.np, s + grain)});
+        }
+    };
+    size_t before0 = 0, before1 = 0;
+    for (size_t w0 = 0; w0 < order.size();) {
+        size_t w1 = w0;
+        uint64_t slots = 0;
+        while (w1 < order.size() && (w1 == w0 || slots + fd[order[w1]].cap <= kWaveSlots)) slots += fd[order[w1++]].cap;
+        for (size_t q = w0; q < w1; ++q) {
+            FragDesc& f = fd[order[q]];
+            for (uint64_t s = 0; s < f.cap; s += (uint64_t)grain * 2, ++f.n_init)
+                items.push_back({order[q], 0, (int64_t)s, (int64_t)std::min<uint64_t>(f.cap, s + grain * 2)});
+        }
+        for (size_t q = w0; q < w1; ++q) {
+            FragDesc& f = fd[order[q]];
+            for (int64_t s = 0; s < f.nb; s += grain, ++f.n_build)
+                items.push_back({order[q], 1, s, std::min<int64_t>(f.nb, s + grain)});
+        }
+        probes(before0, before1);
+        before0 = w0;
+        before1 = w1;
+        w0 = w1;
+    }
+    probes(before0, before1);
     b->empty_frag.assign(n, 0);
     for (int i = 0; i < n; ++i) b->empty_frag[i] = (fd[i].n_build == 0 && fd[i].n_probe == 0);
     FragDesc* dfd;
