@@ -136,8 +136,13 @@ __global__ void assign_kernel(const int64_t* __restrict__ keys, int64_t n, doubl
         uu = uu < 0 ? 0 : (uu > 1 ? 1 : uu);
         leaf[i] = l;
         u[i] = uu;
-        atomicMin(&st[l].lo, (unsigned long long)i);
-        atomicMax(&st[l].hi, (unsigned long long)(i + 1));
+        // Only the ends of a warp's runs of one leaf can be its smallest or
+        // largest index (the lanes hold consecutive samples): the other
+        // lanes' atomics on 1024 leaves took 200 of 240 us for 2^21 samples.
+        const unsigned lane = threadIdx.x & 31, act = __activemask();
+        const int left = __shfl_up_sync(act, l, 1), right = __shfl_down_sync(act, l, 1);
+        if (lane == 0 || left != l) atomicMin(&st[l].lo, (unsigned long long)i);
+        if (lane == 31 || !((act >> (lane + 1)) & 1) || right != l) atomicMax(&st[l].hi, (unsigned long long)(i + 1));
     }
 }
 
@@ -227,11 +232,20 @@ __global__ void __launch_bounds__(CDF_THREADS) root_ls_kernel(const int64_t* __r
         sy += __shfl_xor_sync(0xffffffffu, sy, o);
         sxy += __shfl_xor_sync(0xffffffffu, sxy, o);
     }
+    // One atomic per CTA and sum: one per warp queued up on four addresses.
+    __shared__ double red[4][CDF_THREADS / 32];
     if ((threadIdx.x & 31) == 0) {
-        atomicAdd(&acc[0], sx);
-        atomicAdd(&acc[1], sxx);
-        atomicAdd(&acc[2], sy);
-        atomicAdd(&acc[3], sxy);
+        const int w = threadIdx.x >> 5;
+        red[0][w] = sx;
+        red[1][w] = sxx;
+        red[2][w] = sy;
+        red[3][w] = sxy;
+    }
+    __syncthreads();
+    if (threadIdx.x < 4) {
+        double v = 0;
+        for (int w = 0; w < CDF_THREADS / 32; ++w) v += red[threadIdx.x][w];
+        atomicAdd(&acc[threadIdx.x], v);
     }
 }
 
@@ -923,6 +937,7 @@ int cdf_bin_model(pyg_ctx* ctx, const pyg_cdf* m, int fbits, RJModel* out)
     r.a0 = std::max(0.f, m->a0);
     r.b0 = m->b0;
     r.L = L;
+    r.H = H;
     r.fbits = fbits;
     *out = r;
     return PYG_OK;

@@ -282,6 +282,17 @@ struct RJPartSmem {
     unsigned hot;                      // a bin that held many of the last tile's tuples, else no bin
     int ok;
     long long split[2][MODE == RJ_MODE_RANGE ? RJ_SPLIT_MAX : 1];  // the splitters of this tile and the next
+    // Model bins of 16-byte tuples: the model's tables, where they fit.  A
+    // first pass reads leaves at random: through L1 each lane of a gather is
+    // a tag lookup, in shared memory it is a few bank conflicts (both passes'
+    // first halves of 2^26 x 2^28, theta 1.0: 3.75 -> 2.87 ms; what bounds
+    // them now is shared memory, 76% busy).  Second passes meet the few
+    // leaves of one coarse partition and hit L1.
+    static constexpr bool TABLES = MODE == RJ_MODE_MODEL && !IN8;
+    RJLeaf leaf[TABLES ? RJ_SM_LEAVES : 1];
+    int2 hinfo[TABLES ? RJ_SM_LEAVES : 1];
+    long long hkey[TABLES ? RJ_SM_HEAVY : 1];
+    float hw[TABLES ? RJ_SM_HEAVY : 1];
 };
 __device__ __forceinline__ unsigned rj_range_bin(const long long* sp, int n, long long k)
 {
@@ -390,6 +401,19 @@ __global__ void __launch_bounds__(RJShape<IN8, OUT8, MODE>::THREADS, RJShape<IN8
     const int L = 1 << a.lbits;
     const int tid = threadIdx.x, lane = tid & 31;
     for (int b = tid; b < 2 * BINS; b += T + 32 * NC) (&sm.hist[0][0])[b] = 0;
+    const bool tables = Smem::TABLES && a.model.L <= RJ_SM_LEAVES && a.model.H <= RJ_SM_HEAVY;
+    if constexpr (Smem::TABLES) {
+        if (tables) {
+            for (int l = tid; l < a.model.L; l += T + 32 * NC) {
+                sm.leaf[l] = a.model.leaf[l];
+                if (a.model.H) sm.hinfo[l] = a.model.hinfo[l];
+            }
+            for (int h = tid; h < a.model.H; h += T + 32 * NC) {
+                sm.hkey[h] = a.model.hkey[h];
+                sm.hw[h] = a.model.hw[h];
+            }
+        }
+    }
     if (tid >= T) {
         // ---- control warps; the first one does all but the reservations
         const int ct = tid - T;
@@ -540,7 +564,18 @@ __global__ void __launch_bounds__(RJShape<IN8, OUT8, MODE>::THREADS, RJShape<IN8
                         miss |= (unsigned)(dk >> 32) | (unsigned)(dp >> 32);
                         t[j] = (dk & 0xFFFFFFFFULL) | (dp << 32);
                     }
-                    if constexpr (MODE == RJ_MODE_MODEL)
+                    if constexpr (Smem::TABLES) {
+                        if (tables) {
+                            RJModel m = a.model;
+                            m.leaf = sm.leaf;
+                            m.hinfo = a.model.H ? sm.hinfo : nullptr;
+                            m.hkey = sm.hkey;
+                            m.hw = sm.hw;
+                            bin = rj_bin(rj_model_code(m, key), a.shift, a.mask);
+                        } else {
+                            bin = rj_bin(rj_model_code(a.model, key), a.shift, a.mask);
+                        }
+                    } else if constexpr (MODE == RJ_MODE_MODEL)
                         bin = rj_bin(rj_model_code(a.model, key), a.shift, a.mask);
                     else if constexpr (MODE == RJ_MODE_RANGE)
                         bin = rj_range_bin(sm.split[a.nseg > 1 ? (k & 1) : 0], a.nsplit, key);

@@ -41,6 +41,9 @@ constexpr int RJ_TILE_P = 7936;    // 16-byte tuples in, packed words out: hash 
 constexpr int RJ_TILE_PM = 3968;   //   model and range bins
 constexpr int RJ_TILE_8 = 5376;    // packed words in and out: hash bins
 constexpr int RJ_TILE_8M = 4800;   //   model and range bins
+// Largest model whose tables a first pass keeps in shared memory.
+constexpr int RJ_SM_LEAVES = 1024;
+constexpr int RJ_SM_HEAVY = 512;
 constexpr int RJ_TILE_MIN = 1024;
 // Tile of a pass over n elements: the largest, halved until a pass has about
 // two tiles for each of 148 SMs (small relations would otherwise leave SMs
@@ -95,6 +98,7 @@ struct RJModel {
     float scale = 0;
     float a0 = 0, b0 = 0;
     int L = 0;
+    int H = 0;  // heavy keys
     int fbits = 0;
 };
 
