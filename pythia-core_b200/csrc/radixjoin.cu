@@ -78,6 +78,11 @@ struct RJJoinArgs {
     const void* S;              // 16-byte tuples, or packed words when SP
     const RJItem* items;
     long long nitems;
+    // Items formed on the device (null otherwise): their number, which the
+    // host has not seen (more than nitems, the room for them: nothing is
+    // done), and the partitions' flags (any set: nothing is done).
+    const unsigned long long* total;
+    const unsigned* flags;
     unsigned* next;             // work queue head, zeroed
     int fine_bits;              // the table's slot uses the hash bits below these
     unsigned long long* acc;    // count, build sum, probe sum
@@ -85,6 +90,74 @@ struct RJJoinArgs {
     unsigned long long rk, rp;  // frame of packed build words: key = rk + low half, payload = rp + high half
     unsigned long long sk, sp;  // frame of packed probe words
 };
+
+// The number of items to work on.
+__device__ __forceinline__ long long rj_items(const RJJoinArgs& a)
+{
+    if (!a.total) return a.nitems;
+    unsigned bad = 0;
+    for (int i = 0; i < 8; ++i) bad |= a.flags[i];
+    const unsigned long long n = *a.total;
+    return bad || n > (unsigned long long)a.nitems ? 0 : (long long)n;
+}
+
+// Work items formed on the device: the (build chunk, probe chunk) pairs of
+// every partition with both sides non-empty, in any order of the partitions.
+// Saves the host round trip that reads the counts, builds the items and
+// uploads them: 0.44 ms of the R 2^27 x S 2^30 join.
+struct RJItemArgs {
+    RPDev R, S;
+    int F;
+    unsigned rcap;
+    RJItem* items;
+    unsigned long long room;
+    unsigned long long* total;  // zeroed
+};
+
+constexpr int RJ_ITEM_THREADS = 256;
+
+__global__ void __launch_bounds__(RJ_ITEM_THREADS) rj_items_kernel(RJItemArgs a)
+{
+    __shared__ unsigned long long warp_tot[RJ_ITEM_THREADS / 32], base;
+    const int f = blockIdx.x * RJ_ITEM_THREADS + threadIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    unsigned long long rn = 0, sn = 0, mine = 0;
+    if (f < a.F) {
+        rn = a.R.count[(size_t)f * a.R.stride];
+        sn = a.S.count[(size_t)f * a.S.stride];
+        mine = ((rn + a.rcap - 1) / a.rcap) * ((sn + RJ_SCHUNK - 1) / RJ_SCHUNK);
+    }
+    unsigned long long incl = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+    }
+    if (lane == 31) warp_tot[w] = incl;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned long long all = 0;
+        for (int v = 0; v < RJ_ITEM_THREADS / 32; ++v) {
+            const unsigned long long t = warp_tot[v];
+            warp_tot[v] = all;
+            all += t;
+        }
+        base = all ? atomicAdd(a.total, all) : 0;
+    }
+    __syncthreads();
+    if (!mine) return;
+    unsigned long long at = base + warp_tot[w] + incl - mine;
+    if (at + mine > a.room) return;  // the host forms the items then
+    const unsigned long long r0 = a.R.start[f], s0 = a.S.start[f];
+    for (unsigned long long r = 0; r < rn; r += a.rcap)
+        for (unsigned long long s = 0; s < sn; s += RJ_SCHUNK) {
+            RJItem it;
+            it.r0 = r0 + r;
+            it.s0 = s0 + s;
+            it.rn = (unsigned)min((unsigned long long)a.rcap, rn - r);
+            it.sn = (unsigned)min((unsigned long long)RJ_SCHUNK, sn - s);
+            a.items[at++] = it;
+        }
+}
 
 // Tuple i of a partitioned relation as (key, payload).
 template <bool PACKED>
@@ -138,6 +211,7 @@ __global__ void __launch_bounds__(RJ_JOIN_THREADS, RJ_JOIN_BLOCKS) rj_join_kerne
     __shared__ unsigned long long side_cnt, side_sum;
     ulonglong2* T2 = reinterpret_cast<ulonglong2*>(rj_table);  // UNIQUE slots
     ulonglong4* T4 = reinterpret_cast<ulonglong4*>(rj_table);  // counted slots
+    const long long nitems = rj_items(a);
     uint64_t cnt = 0, bsum = 0, psum = 0;
     bool dup = false;
     // One item of look-ahead: while this CTA works on an item, the next
@@ -149,9 +223,9 @@ __global__ void __launch_bounds__(RJ_JOIN_THREADS, RJ_JOIN_BLOCKS) rj_join_kerne
         if (threadIdx.x == 0) {
             item_cur = item_next;
             side_cnt = side_sum = 0;
-            if (item_cur < a.nitems) {
+            if (item_cur < nitems) {
                 item_next = (long long)atomicAdd(a.next, 1u);
-                if (item_next < a.nitems) {
+                if (item_next < nitems) {
                     const RJItem nx = a.items[item_next];
                     rj_prefetch_l2((const char*)a.R + nx.r0 * RB, (unsigned long long)nx.rn * RB);
                     rj_prefetch_l2((const char*)a.S + nx.s0 * SB, (unsigned long long)min(nx.sn, 4096u) * SB);
@@ -164,7 +238,7 @@ __global__ void __launch_bounds__(RJ_JOIN_THREADS, RJ_JOIN_BLOCKS) rj_join_kerne
         }
         __syncthreads();
         const long long it = item_cur;
-        if (it >= a.nitems) break;
+        if (it >= nitems) break;
         const RJItem item = a.items[it];
         // Build: linear probing with 64-bit shared-memory CAS.  At most
         // TS / 2 tuples per item, so a free slot always exists.
@@ -304,6 +378,7 @@ __global__ void __launch_bounds__(RJ32_THREADS, RJ32_BLOCKS) rj_join32_kernel(RJ
     __shared__ long long item_cur, item_next;
     const unsigned long long* Rw = reinterpret_cast<const unsigned long long*>(a.R);
     const unsigned long long* Sw = reinterpret_cast<const unsigned long long*>(a.S);
+    const long long nitems = rj_items(a);
     uint64_t cnt = 0, bsum = 0, psum = 0;  // matches, build and probe payload offsets
     bool dup = false;
     if (threadIdx.x == 0) item_next = (long long)atomicAdd(a.next, 1u);
@@ -311,9 +386,9 @@ __global__ void __launch_bounds__(RJ32_THREADS, RJ32_BLOCKS) rj_join32_kernel(RJ
         __syncthreads();  // previous item done with the table and item slots
         if (threadIdx.x == 0) {
             item_cur = item_next;
-            if (item_cur < a.nitems) {
+            if (item_cur < nitems) {
                 item_next = (long long)atomicAdd(a.next, 1u);
-                if (item_next < a.nitems) {
+                if (item_next < nitems) {
                     const RJItem nx = a.items[item_next];
                     rj_prefetch_l2(Rw + nx.r0, (unsigned long long)nx.rn * 8);
                     rj_prefetch_l2(Sw + nx.s0, (unsigned long long)min(nx.sn, RJ32_PREFETCH) * 8);
@@ -325,7 +400,7 @@ __global__ void __launch_bounds__(RJ32_THREADS, RJ32_BLOCKS) rj_join32_kernel(RJ
             T2[i] = make_ulonglong2(kEmptyWord, kEmptyWord);
         __syncthreads();
         const long long it = item_cur;
-        if (it >= a.nitems) break;
+        if (it >= nitems) break;
         const RJItem item = a.items[it];
         // Build: one 64-bit CAS per word; a chunk fills at most half the
         // table, so a free slot always exists.
@@ -500,37 +575,14 @@ int radix_join16(pyg_ctx* ctx, const void* Rv, int64_t nR, const void* Sv, int64
             side[s].mid = tm.on ? tm.ev[6 + 2 * s] : nullptr;
             side[s].done = tm.on ? tm.ev[2 + s] : nullptr;
         }
-        rc = rp_partition_sides(ctx, side, 2, FB, two, flags, hflags, tm.on ? tm.ev[1] : nullptr, true);
-        R1 = side[0].P1;
-        R2 = side[0].P2;
-        S1 = side[1].P1;
-        S2 = side[1].P2;
-        if (rc) break;
-        const RJLayout& LR = side[0].L;
-        const RJLayout& LS = side[1].L;
-
-        // 3. Join: distinct build keys first (16-byte slots); on a repeated
-        // key, again with counted 32-byte slots and smaller build chunks.
         unsigned long long* acc = ctx->dcounters + 8;
-        unsigned* next = (unsigned*)(ctx->dcounters + 200);  // word 200: queue head, word 201: dup flag
+        // Words 200: queue head, 201: dup flag, 202: items formed on the device.
+        unsigned* next = (unsigned*)(ctx->dcounters + 200);
         unsigned* dupf = (unsigned*)(ctx->dcounters + 201);
-        std::vector<unsigned long long> rstart(LR.fstart.begin(), LR.fstart.begin() + F);
-        std::vector<unsigned long long> sstart(LS.fstart.begin(), LS.fstart.begin() + F);
-        std::vector<RJItem> items;
-        // Both relations packed in one key frame: the 32-bit-offset join
-        // (distinct build keys; a repeated key falls back to the counted
-        // join below, which decodes the words).
-        const bool same_frame = LR.packed && LS.packed && LR.kbase == LS.kbase;
-        for (int pass = 0; pass < 2; ++pass) {
-            const bool unique = pass == 0;
-            const bool j32 = unique && same_frame;
-            make_items(LR.count, LS.count, rstart, sstart,
-                       j32 ? RJ32_RCAP : (unique ? RJ_RCAP_UNIQUE : RJ_RCAP_COUNTED), items);
-            if (items.empty()) break;
-            dfree(ctx, ditems);
-            ditems = nullptr;
-            if ((rc = dalloc(ctx, (void**)&ditems, items.size() * sizeof(RJItem)))) break;
-            if ((rc = stage_h2d(ctx, ditems, items.data(), items.size() * sizeof(RJItem)))) break;
+        // Launches the join kernel of the partitions' formats on `items`.
+        auto join = [&](bool unique, const RJItem* items, long long nitems, const unsigned long long* total) -> int {
+            const RJLayout &LR = side[0].L, &LS = side[1].L;
+            const bool j32 = unique && LR.packed && LS.packed && LR.kbase == LS.kbase;
             void* fn = j32 ? (void*)rj_join32_kernel
                            : (unique ? join_fn<true>(LR.packed, LS.packed) : join_fn<false>(LR.packed, LS.packed));
             const int smem = j32 ? RJ32_TABLE_BYTES : RJ_TABLE_BYTES;
@@ -540,10 +592,12 @@ int radix_join16(pyg_ctx* ctx, const void* Rv, int64_t nR, const void* Sv, int64
             PYG_CUDA(cudaMemsetAsync(acc, 0, 3 * 8, ctx->stream));
             PYG_CUDA(cudaMemsetAsync(next, 0, 16, ctx->stream));
             RJJoinArgs ja;
-            ja.R = two ? R2 : R1;
-            ja.S = two ? S2 : S1;
-            ja.items = ditems;
-            ja.nitems = (long long)items.size();
+            ja.R = two ? side[0].P2 : side[0].P1;
+            ja.S = two ? side[1].P2 : side[1].P1;
+            ja.items = items;
+            ja.nitems = nitems;
+            ja.total = total;
+            ja.flags = flags;
             ja.next = next;
             ja.fine_bits = FB;
             ja.acc = acc;
@@ -552,21 +606,81 @@ int radix_join16(pyg_ctx* ctx, const void* Rv, int64_t nR, const void* Sv, int64
             ja.rp = LR.pbase;
             ja.sk = LS.kbase;
             ja.sp = LS.pbase;
-            const unsigned grid = (unsigned)std::min<long long>((long long)ctx->sm_count * per_sm, ja.nitems);
+            const unsigned grid = (unsigned)std::min<long long>((long long)ctx->sm_count * per_sm, nitems);
             if (unique) tm.mark(ctx, 9);
             void* args[] = {&ja};
             PYG_CUDA(cudaLaunchKernel(fn, dim3(grid), dim3(threads), args, smem, ctx->stream));
             PYG_LAUNCHED(ctx);
             PYG_CUDA(cudaMemcpyAsync(h, acc, 3 * 8, cudaMemcpyDeviceToHost, ctx->stream));
-            PYG_CUDA(cudaMemcpyAsync(h + 3, next, 16, cudaMemcpyDeviceToHost, ctx->stream));
+            PYG_CUDA(cudaMemcpyAsync(h + 3, next, 24, cudaMemcpyDeviceToHost, ctx->stream));
+            return PYG_OK;
+        };
+        // The join of distinct build keys follows the passes without the
+        // host: its items are formed on the device.  Room for an item per
+        // partition and whole chunk of either side; a partition that is cut
+        // on both sides can need more, and then the host forms them.
+        const long long room = F + nS / RJ_SCHUNK + nR / RJ32_RCAP + 1024;
+        bool settled = false, only_dup = false;
+        RPAfter after;
+        after.enqueue = [&](const RPDev* dev) -> int {
+            const RJLayout &LR = side[0].L, &LS = side[1].L;
+            int r;
+            if ((r = dalloc(ctx, (void**)&ditems, (size_t)room * sizeof(RJItem)))) return r;
+            RJItemArgs ia;
+            ia.R = dev[0];
+            ia.S = dev[1];
+            ia.F = F;
+            ia.rcap = LR.packed && LS.packed && LR.kbase == LS.kbase ? RJ32_RCAP : RJ_RCAP_UNIQUE;
+            ia.items = ditems;
+            ia.room = (unsigned long long)room;
+            ia.total = ctx->dcounters + 202;
+            PYG_CUDA(cudaMemsetAsync(ia.total, 0, 8, ctx->stream));
+            rj_items_kernel<<<(F + RJ_ITEM_THREADS - 1) / RJ_ITEM_THREADS, RJ_ITEM_THREADS, 0, ctx->stream>>>(ia);
+            PYG_LAUNCHED(ctx);
+            if ((r = join(true, ditems, room, ia.total))) return r;
+            tm.mark(ctx, 4);
+            return PYG_OK;
+        };
+        after.settled = [&]() -> bool {
+            bool clean = h[5] <= (unsigned long long)room;
+            for (int i = 0; i < 8; ++i) clean &= (i & 3) == 3 || hflags[i] == 0;
+            only_dup = clean && (unsigned)h[4] != 0;
+            settled = clean && !only_dup;
+            return settled;
+        };
+        rc = rp_partition_sides(ctx, side, 2, FB, two, flags, hflags, tm.on ? tm.ev[1] : nullptr, true, &after);
+        R1 = side[0].P1;
+        R2 = side[0].P2;
+        S1 = side[1].P1;
+        S2 = side[1].P2;
+        if (rc) break;
+        const RJLayout& LR = side[0].L;
+        const RJLayout& LS = side[1].L;
+        for (int j = 0; j < 3; ++j) out[j] = h[j];
+
+        // 3. Where that did not settle it: items from the host, distinct build
+        // keys first (16-byte slots; 8-byte ones where both relations are
+        // packed in one key frame); on a repeated key, again with counted
+        // 32-byte slots and smaller build chunks.
+        const bool same_frame = LR.packed && LS.packed && LR.kbase == LS.kbase;
+        for (int pass = only_dup ? 1 : 0; !settled && pass < 2; ++pass) {
+            const bool unique = pass == 0;
+            std::vector<RJItem> items;
+            out[0] = out[1] = out[2] = 0;
+            make_items(LR.count, LS.count, LR.fstart, LS.fstart,
+                       unique && same_frame ? RJ32_RCAP : (unique ? RJ_RCAP_UNIQUE : RJ_RCAP_COUNTED), items);
+            if (items.empty()) break;
+            dfree(ctx, ditems);
+            ditems = nullptr;
+            if ((rc = dalloc(ctx, (void**)&ditems, items.size() * sizeof(RJItem)))) break;
+            if ((rc = stage_h2d(ctx, ditems, items.data(), items.size() * sizeof(RJItem)))) break;
+            if ((rc = join(unique, ditems, (long long)items.size(), nullptr))) break;
             PYG_CUDA(cudaStreamSynchronize(ctx->stream));
-            out[0] = h[0];
-            out[1] = h[1];
-            out[2] = h[2];
+            for (int j = 0; j < 3; ++j) out[j] = h[j];
             if (!unique || (unsigned)h[4] == 0) break;
         }
         if (rc) break;
-        tm.mark(ctx, 4);
+        if (!settled) tm.mark(ctx, 4);
         if (stats) {
             cudaEventSynchronize(tm.ev[4]);
             // Histograms of both relations, then the build side's passes

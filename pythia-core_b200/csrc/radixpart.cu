@@ -111,24 +111,36 @@ __global__ void rj_hist_sum_kernel(const unsigned* __restrict__ part, int nrow, 
     hist[b] = sum;
 }
 
-// Tiles of `tile` elements per segment, as an exclusive prefix (one thread;
-// at most 2^8 segments): tiles[C] is the pass's tile count.  Counts are
-// first clamped to their region's capacity, so a region that overflowed
-// (its result is discarded and redone) is never read past its end.
-__global__ void rj_tile_prefix_kernel(const unsigned long long* __restrict__ cursor, int cstride,
-                                      unsigned long long* __restrict__ count, const unsigned long long* __restrict__ cap,
-                                      int C, int tile, unsigned long long* __restrict__ tiles)
+// Tiles of `tile` elements per segment, as an exclusive prefix (one CTA, one
+// thread per segment; at most 2^9 segments): tiles[C] is the pass's tile
+// count.  Counts are first clamped to their region's capacity, so a region
+// that overflowed (its result is discarded and redone) is never read past its
+// end.
+__global__ void __launch_bounds__(RJ_LMAX) rj_tile_prefix_kernel(const unsigned long long* __restrict__ cursor, int cstride,
+                                                                 unsigned long long* __restrict__ count,
+                                                                 const unsigned long long* __restrict__ cap, int C,
+                                                                 int tile, unsigned long long* __restrict__ tiles)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+    __shared__ unsigned long long warp_tot[RJ_LMAX / 32];
+    const int c = threadIdx.x, lane = c & 31, w = c >> 5;
     unsigned long long t = 0;
-    tiles[0] = 0;
-    for (int c = 0; c < C; ++c) {
+    if (c < C) {
         const unsigned long long reached = cursor[(size_t)c * cstride];
         const unsigned long long n = reached < cap[c] ? reached : cap[c];
         count[c] = n;
-        t += (n + tile - 1) / tile;
-        tiles[c + 1] = t;
+        t = (n + tile - 1) / tile;
     }
+    unsigned long long incl = t;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+    }
+    if (lane == 31) warp_tot[w] = incl;
+    __syncthreads();
+    for (int v = 0; v < w; ++v) incl += warp_tot[v];
+    if (c == 0) tiles[0] = 0;
+    if (c < C) tiles[c + 1] = incl;
 }
 
 // ---------------------------------------------------------------------------
@@ -713,10 +725,11 @@ void layout_exact(const std::vector<unsigned long long>& h, int64_t n, int C, in
     L.p1 = L.p2 = L.fstart[F];
 }
 
-unsigned long long sampled_cap(unsigned long long c, long long step, unsigned long long extra)
+// Capacity of a region that c of the samples fell into (rounded up).
+static inline unsigned long long sampled_cap(unsigned long long c, long long step, unsigned long long extra)
 {
-    const double x = (double)c;
-    return (unsigned long long)std::ceil((x + 6.0 * std::sqrt(x) + 8.0) * (double)step) + extra;
+    return (c + 8) * (unsigned long long)step + (unsigned long long)(long long)(6.0 * std::sqrt((double)c) * (double)step) + 1 +
+           extra;
 }
 
 void layout_sampled(const std::vector<unsigned long long>& sc, long long step, int64_t n, int C, int sub, RJLayout& L,
@@ -788,18 +801,23 @@ bool common_key_frame(const long long* mm0, bool exact0, const long long* mm1, b
 
 int upload_layout(pyg_ctx* ctx, const RJLayout& L, const RJSideDev& d, int F, int C, int64_t n)
 {
+    // fstart, fcap, cstart and ccap are adjacent on the device, and so are
+    // tiles2 and whole: two copies.
     int rc;
-    if ((rc = stage_h2d(ctx, d.fstart, L.fstart.data(), (size_t)(F + 1) * 8))) return rc;
-    if ((rc = stage_h2d(ctx, d.cstart, L.cstart.data(), (size_t)(C + 1) * 8))) return rc;
-    if (L.sampled && (rc = stage_h2d(ctx, d.fcap, L.fcap.data(), (size_t)F * 8))) return rc;
-    if (L.sampled || L.packed) {
-        if ((rc = stage_h2d(ctx, d.ccap, L.ccap.data(), (size_t)C * 8))) return rc;
-    } else if ((rc = stage_h2d(ctx, d.tiles2, L.tiles2.data(), (size_t)(C + 1) * 8))) {
-        return rc;
-    }
+    std::vector<unsigned long long> m((size_t)(F + 1) + F + (C + 1) + C, 0);
+    unsigned long long* p = m.data();
+    memcpy(p, L.fstart.data(), (size_t)(F + 1) * 8);
+    if (L.sampled) memcpy(p + F + 1, L.fcap.data(), (size_t)F * 8);
+    memcpy(p + 2 * F + 1, L.cstart.data(), (size_t)(C + 1) * 8);
+    if (L.sampled || L.packed) memcpy(p + 2 * F + C + 2, L.ccap.data(), (size_t)C * 8);
+    if ((rc = stage_h2d(ctx, d.fstart, p, m.size() * 8))) return rc;
+    std::vector<unsigned long long> t((size_t)(C + 1) + 4, 0);
+    if (!L.sampled && !L.packed) memcpy(t.data(), L.tiles2.data(), (size_t)(C + 1) * 8);
+    t[C + 2] = (unsigned long long)n;
+    t[C + 4] = (unsigned long long)((n + L.tile1 - 1) / L.tile1);
+    if ((rc = stage_h2d(ctx, d.tiles2, t.data(), t.size() * 8))) return rc;
     PYG_CUDA(cudaMemsetAsync(d.cur1, 0, ((size_t)C * RJ_CURSOR_STRIDE + F) * 8, ctx->stream));  // cur1 and cur2 are adjacent
-    const unsigned long long w[4] = {0, (unsigned long long)n, 0, (unsigned long long)((n + L.tile1 - 1) / L.tile1)};
-    return stage_h2d(ctx, d.whole, w, sizeof(w));
+    return PYG_OK;
 }
 
 // Runs the partition pass(es) of one relation into P1 (and P2).
@@ -845,7 +863,7 @@ int run_passes(pyg_ctx* ctx, const longlong2* in, int64_t n, const RJLayout& L, 
     if (L.sampled || L.packed) {
         // Second-pass segments are the first pass's regions, filled to the
         // counts its cursors reached; the tile prefix is formed on the device.
-        rj_tile_prefix_kernel<<<1, 32, 0, ctx->stream>>>(d.cur1, RJ_CURSOR_STRIDE, d.count1, d.ccap, C,
+        rj_tile_prefix_kernel<<<1, RJ_LMAX, 0, ctx->stream>>>(d.cur1, RJ_CURSOR_STRIDE, d.count1, d.ccap, C,
                                                           L.tile2, d.tiles2);
         PYG_LAUNCHED(ctx);
         p.seg_count = d.count1;
@@ -933,7 +951,7 @@ int hist_launch_range(pyg_ctx* ctx, const longlong2* in, int64_t n, int64_t step
 }
 
 int rp_partition_sides(pyg_ctx* ctx, RPSide* sd, int ns, int FB, bool two, unsigned* flags, unsigned* hflags,
-                       cudaEvent_t hist_done, bool share_key_frame)
+                       cudaEvent_t hist_done, bool share_key_frame, const RPAfter* after)
 {
     // Coarse bits of the first of two passes.  Unpacked layouts split FB
     // evenly (2048-tuple tiles); packed layouts keep the second pass at 2^8
@@ -1033,6 +1051,17 @@ int rp_partition_sides(pyg_ctx* ctx, RPSide* sd, int ns, int FB, bool two, unsig
         }
         if (rc) break;
         PYG_CUDA(cudaMemcpyAsync(hflags, flags, (size_t)16 * ns, cudaMemcpyDeviceToHost, ctx->stream));
+        if (after) {
+            RPDev dev[2];
+            for (int s = 0; s < ns; ++s) {
+                dev[s].start = d[s].fstart;
+                dev[s].count = two ? d[s].cur2 : d[s].cur1;
+                dev[s].stride = two ? 1 : RJ_CURSOR_STRIDE;
+            }
+            if ((rc = after->enqueue(dev))) break;
+            PYG_CUDA(cudaStreamSynchronize(ctx->stream));
+            if (after->settled()) break;
+        }
         for (int s = 0; s < ns; ++s)
             if (sd[s].L.sampled)
                 PYG_CUDA(cudaMemcpyAsync(hh_at(s), two ? d[s].cur2 : d[s].cur1,

@@ -26,6 +26,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <functional>
 #include <vector>
 
 #include "pyg_internal.cuh"
@@ -268,6 +269,25 @@ struct RPSide {
     bool overflowed = false;
 };
 
+// One relation's partitions on the device, valid in stream order: partition
+// f starts at start[f] and holds count[f * stride] elements (more than its
+// region holds if it overflowed: the relation's flags then say so).
+struct RPDev {
+    const unsigned long long* start;
+    const unsigned long long* count;
+    int stride;
+};
+
+// What a caller does with the partitions before the host has seen their
+// counts: enqueue launches it behind the passes (its kernels must do nothing
+// when a relation's flags are set), settled is asked after the stream was
+// synchronised and the flags are on the host; true: the answer stands, and
+// the counts and the redo are not needed.
+struct RPAfter {
+    std::function<int(const RPDev*)> enqueue;
+    std::function<bool()> settled;
+};
+
 // Partitions one or two relations with the same bits: both histograms, one
 // host round trip, both relations' passes (the second relation's layout is
 // formed while the first one's passes run), one more round trip for the
@@ -278,8 +298,9 @@ struct RPSide {
 // hist_done (optional) is recorded after the histograms.
 // share_key_frame: pack both relations with one key frame when their key
 // ranges fit one (a redone relation gets its own frame).
+// after (optional): work on the partitions that needs no host round trip.
 int rp_partition_sides(pyg_ctx* ctx, RPSide* sd, int ns, int FB, bool two, unsigned* flags, unsigned* hflags,
-                       cudaEvent_t hist_done, bool share_key_frame = false);
+                       cudaEvent_t hist_done, bool share_key_frame = false, const RPAfter* after = nullptr);
 
 // Partitions one relation into 2^FB partitions (hash bits, or ranges when
 // csplit is set; two passes when `two`): histogram (sampled when allowed

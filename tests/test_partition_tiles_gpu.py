@@ -42,3 +42,21 @@ def test_unpacked_tile_edges(ctx, torch_cuda, bits, nS):
     got = ctx.hashjoin_agg(dev_rel(torch_cuda, R, [I64, I64]), [0], dev_rel(torch_cuda, S, [I64, I64]), [0],
                            [(0, 1), (1, 1)], pyg.JOIN_RADIX, bits)
     assert got == (nS, [sb, int(S["c1"].sum())])
+
+
+@pytest.mark.parametrize("dup", [False, True])
+def test_items_beyond_the_device_list(ctx, torch_cuda, dup):
+    """Two partitions cut into many chunks on both sides need more work items
+    than the device forms: the host does."""
+    n = 2_000_003
+    R, S, sb, sp = relations(n, n, 0.0, 5, 11)
+    if dup:  # one build key twice
+        R["c0"][7] = R["c0"][8]
+        hit = S["c0"] == R["c0"][8]
+        lost = S["c0"] == R["c1"][7] // 7
+        sb = int((S["c0"][~lost] * 7).sum() + hit.sum() * int(R["c1"][7]))
+        sp = int(S["c1"][~lost].sum() + S["c1"][hit].sum())
+        n += int(hit.sum()) - int(lost.sum())
+    got = ctx.hashjoin_agg(dev_rel(torch_cuda, R, [I64, I64]), [0], dev_rel(torch_cuda, S, [I64, I64]), [0],
+                           [(0, 1), (1, 1)], pyg.JOIN_RADIX, 1)
+    assert got == (n, [sb, sp])
