@@ -8,8 +8,8 @@
 //                  the radix operators' bulk-copy partitioner (radixpart.cu,
 //                  two passes above 2^8 ranges): splitter-search bins, or,
 //                  for a learned model, the model's own bins (rj_model_bin,
-//                  the same ranges without a search), whose intermediates
-//                  are packed 8-byte words when the key and payload ranges
+//                  the same ranges without a search).  The intermediates are
+//                  packed 8-byte words when the key and payload ranges
 //                  allow; the merge decodes them on load.
 //   3. sort+merge  persistent CTAs take (range, build chunk, probe chunk)
 //                  items.  A range whose splitters bound it to at most
@@ -321,30 +321,29 @@ int mpsm16_agg(pyg_ctx* ctx, const void* Rv, int64_t nR, const void* Sv, int64_t
         unsigned* flags = (unsigned*)(ctx->dcounters + 208);
         unsigned* hflags = (unsigned*)ctx->pinned + 96;
         RJLayout LR, LS;
-        if (model) {
-            // Bins from the model: no splitter search in the histograms or
-            // passes, and both relations' histograms in one round trip.
-            RPSide sd[2];
-            sd[0].in = R;
-            sd[0].n = nR;
-            sd[1].in = S;
-            sd[1].n = nS;
-            sd[0].model = sd[1].model = model;
-            // One bin function for both passes: the intermediates can be
-            // packed words whatever split of bits the passes take.
-            sd[0].allow_pack = sd[1].allow_pack = true;
-            rc = rp_partition_sides(ctx, sd, 2, FB, two, flags, hflags, nullptr);
-            R1 = sd[0].P1;
-            R2 = sd[0].P2;
-            S1 = sd[1].P1;
-            S2 = sd[1].P2;
-            if (rc) break;
-            LR = std::move(sd[0].L);
-            LS = std::move(sd[1].L);
-        } else {
-            if ((rc = rp_partition(ctx, R, nR, FB, two, true, cs, fs, LR, &R1, &R2, flags, hflags))) break;
-            if ((rc = rp_partition(ctx, S, nS, FB, two, true, cs, fs, LS, &S1, &S2, flags, hflags))) break;
+        // Bins from the model or the splitters, and both relations'
+        // histograms in one round trip.  Either way one bin function (or one
+        // split of the bits) serves both passes, so the intermediates are
+        // packed words where the key and payload ranges allow.
+        RPSide sd[2];
+        for (int s = 0; s < 2; ++s) {
+            sd[s].in = s ? S : R;
+            sd[s].n = s ? nS : nR;
+            sd[s].allow_pack = true;
+            sd[s].model = model;
+            if (!model) {
+                sd[s].csplit = cs;
+                sd[s].fsplit = fs;
+            }
         }
+        rc = rp_partition_sides(ctx, sd, 2, FB, two, flags, hflags, nullptr);
+        R1 = sd[0].P1;
+        R2 = sd[0].P2;
+        S1 = sd[1].P1;
+        S2 = sd[1].P2;
+        if (rc) break;
+        LR = std::move(sd[0].L);
+        LS = std::move(sd[1].L);
         cudaEventRecord(ev[1], ctx->stream);
         if (sizes) *sizes = LS.count;
         // Items: every (build chunk, probe chunk) pair of each range.  Range

@@ -334,7 +334,7 @@ __device__ __forceinline__ void rj_load_split(const RJPass& a, long long* dst, i
 __global__ void __launch_bounds__(1024) rj_hist_range_kernel(const longlong2* __restrict__ in, int64_t n, int64_t step,
                                                              int CB, int sub, const long long* __restrict__ csplit,
                                                              const long long* __restrict__ fsplit,
-                                                             unsigned* __restrict__ part)
+                                                             unsigned* __restrict__ part, long long* __restrict__ mm)
 {
     extern __shared__ __align__(16) unsigned char rj_hr_raw[];
     const int F = 1 << (CB + sub), C = 1 << CB, L = 1 << sub;
@@ -344,12 +344,33 @@ __global__ void __launch_bounds__(1024) rj_hist_range_kernel(const longlong2* __
     for (int i = threadIdx.x; i < C - 1; i += blockDim.x) cs[i] = csplit[i];
     __syncthreads();
     const int64_t m = (n + step - 1) / step;
+    long long kmin = LLONG_MAX, kmax = LLONG_MIN, pmin = LLONG_MAX, pmax = LLONG_MIN;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < m; i += stride) {
-        const long long k = __ldcs(&in[i * step]).x;
+        const longlong2 t = __ldcs(&in[i * step]);
+        const long long k = t.x;
+        kmin = min(kmin, t.x);
+        kmax = max(kmax, t.x);
+        pmin = min(pmin, t.y);
+        pmax = max(pmax, t.y);
         unsigned f = rj_range_bin(cs, C - 1, k);
         if (sub) f = (f << sub) | rj_range_bin(fsplit + ((long long)f << sub), L - 1, k);
         atomicAdd(&h[f], 1u);
+    }
+    if (mm) {  // key and payload ranges of the tuples read
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            kmin = min(kmin, __shfl_xor_sync(0xffffffffu, kmin, o));
+            kmax = max(kmax, __shfl_xor_sync(0xffffffffu, kmax, o));
+            pmin = min(pmin, __shfl_xor_sync(0xffffffffu, pmin, o));
+            pmax = max(pmax, __shfl_xor_sync(0xffffffffu, pmax, o));
+        }
+        if ((threadIdx.x & 31) == 0) {
+            atomicMin(&mm[0], kmin);
+            atomicMax(&mm[1], kmax);
+            atomicMin(&mm[2], pmin);
+            atomicMax(&mm[3], pmax);
+        }
     }
     __syncthreads();
     unsigned* row = part + (size_t)blockIdx.x * F;
@@ -826,8 +847,8 @@ int run_passes(pyg_ctx* ctx, const longlong2* in, int64_t n, const RJLayout& L, 
                const long long* fsplit, unsigned* frame, cudaEvent_t between, const RJModel* model)
 {
     const int C = 1 << CB, sub = FB - CB;
-    if (L.packed && (!frame || csplit || (two && sub > 8))) {
-        set_error("partition: packed layouts need a frame flag, hash bins and at most 2^8 second-pass bins");
+    if (L.packed && (!frame || (two && sub > 8))) {
+        set_error("partition: packed layouts need a frame flag and at most 2^8 second-pass bins");
         return PYG_ERR_ARG;
     }
     RJPass p;
@@ -928,7 +949,7 @@ int hist_launch(pyg_ctx* ctx, const longlong2* in, int64_t n, int64_t step, int 
 }
 
 int hist_launch_range(pyg_ctx* ctx, const longlong2* in, int64_t n, int64_t step, int CB, int sub,
-                      const long long* csplit, const long long* fsplit, unsigned long long* hist)
+                      const long long* csplit, const long long* fsplit, unsigned long long* hist, long long* mm)
 {
     const int F = 1 << (CB + sub);
     const size_t hsm = (size_t)RJ_SPLIT_MAX * 8 + (size_t)4 * F;
@@ -942,7 +963,11 @@ int hist_launch_range(pyg_ctx* ctx, const longlong2* in, int64_t n, int64_t step
     unsigned* part = nullptr;
     int rc;
     if ((rc = dalloc(ctx, (void**)&part, (size_t)grid * F * 4))) return rc;
-    rj_hist_range_kernel<<<grid, 1024, hsm, ctx->stream>>>(in, n, step, CB, sub, csplit, fsplit, part);
+    if (mm) {
+        rj_mm_init_kernel<<<1, 32, 0, ctx->stream>>>(mm);
+        PYG_LAUNCHED(ctx);
+    }
+    rj_hist_range_kernel<<<grid, 1024, hsm, ctx->stream>>>(in, n, step, CB, sub, csplit, fsplit, part, mm);
     PYG_LAUNCHED(ctx);
     rj_hist_sum_kernel<<<(F + 255) / 256, 256, 0, ctx->stream>>>(part, grid, F, hist);
     PYG_LAUNCHED(ctx);
@@ -984,7 +1009,8 @@ int rp_partition_sides(pyg_ctx* ctx, RPSide* sd, int ns, int FB, bool two, unsig
     auto hist_of = [&](int s, int64_t st) {
         if (sd[s].csplit) {
             const int cb = coarse_bits(false);
-            return hist_launch_range(ctx, sd[s].in, sd[s].n, st, cb, FB - cb, sd[s].csplit, sd[s].fsplit, hist_at(s));
+            return hist_launch_range(ctx, sd[s].in, sd[s].n, st, cb, FB - cb, sd[s].csplit, sd[s].fsplit, hist_at(s),
+                                     sd[s].allow_pack ? (long long*)(hist_at(s) + F) : nullptr);
         }
         return hist_launch(ctx, sd[s].in, sd[s].n, st, FB, hist_at(s),
                            sd[s].allow_pack ? (long long*)(hist_at(s) + F) : nullptr, sd[s].model);
@@ -994,13 +1020,12 @@ int rp_partition_sides(pyg_ctx* ctx, RPSide* sd, int ns, int FB, bool two, unsig
     auto form = [&](int s, const unsigned long long* h, int64_t st, bool exact, const unsigned long long* kb) {
         RJLayout& L = sd[s].L;
         const long long* mm = (const long long*)(h + F);
-        const bool pack =
-            sd[s].allow_pack && !sd[s].csplit && pack_frame(mm[0], mm[1], mm[2], mm[3], exact, L, kb);
-        CBs[s] = coarse_bits(pack);
+        const bool pack = sd[s].allow_pack && pack_frame(mm[0], mm[1], mm[2], mm[3], exact, L, kb);
+        CBs[s] = coarse_bits(pack && !sd[s].csplit);  // the coarse splitters fix the split of range bins
         const int C = 1 << CBs[s], sub = FB - CBs[s];
         std::vector<unsigned long long> hv(h, h + F);
-        if (exact) layout_exact(hv, sd[s].n, C, sub, L, pack, sd[s].model != nullptr);
-        else layout_sampled(hv, st, sd[s].n, C, sub, L, pack, sd[s].model != nullptr);
+        if (exact) layout_exact(hv, sd[s].n, C, sub, L, pack, sd[s].model || sd[s].csplit);
+        else layout_sampled(hv, st, sd[s].n, C, sub, L, pack, sd[s].model || sd[s].csplit);
         d[s].carve(meta + (size_t)s * per, F, C);
     };
     auto launch = [&](int s) {
@@ -1110,36 +1135,6 @@ int rp_partition_sides(pyg_ctx* ctx, RPSide* sd, int ns, int FB, bool two, unsig
             sd[s].P1 = sd[s].P2 = nullptr;
         }
     }
-    return rc;
-}
-
-int rp_partition(pyg_ctx* ctx, const longlong2* in, int64_t n, int FB, bool two, bool allow_sample,
-                 const long long* csplit, const long long* fsplit, RJLayout& L, void** P1, void** P2,
-                 unsigned* flags, unsigned* hflags, float* hist_ms, int64_t* hist_tuples)
-{
-    RPSide s;
-    s.in = in;
-    s.n = n;
-    s.allow_sample = allow_sample;
-    s.csplit = csplit;
-    s.fsplit = fsplit;
-    cudaEvent_t e0 = nullptr, e1 = nullptr;
-    if (hist_ms) {
-        cudaEventCreate(&e0);
-        cudaEventCreate(&e1);
-        cudaEventRecord(e0, ctx->stream);
-    }
-    const int rc = rp_partition_sides(ctx, &s, 1, FB, two, flags, hflags, e1);
-    if (hist_ms) {
-        *hist_ms = 0.f;
-        if (!rc) cudaEventElapsedTime(hist_ms, e0, e1);
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
-    }
-    if (hist_tuples) *hist_tuples = s.hist_tuples;
-    L = std::move(s.L);
-    *P1 = s.P1;
-    *P2 = s.P2;
     return rc;
 }
 

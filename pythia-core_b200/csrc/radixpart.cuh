@@ -160,7 +160,7 @@ struct RJLayout {
 
 // Exact layout of n tuples from exact per-fine-partition counts h (F = h.size()).
 // pack: regions rounded up to an even number of words (packed layouts).
-// model: the passes' bins are a learned model's.
+// model: the passes' bins are a learned model's or key ranges.
 void layout_exact(const std::vector<unsigned long long>& h, int64_t n, int C, int sub, RJLayout& L,
                   bool pack = false, bool model = false);
 // Sampled layout from the counts sc of every step-th tuple: each region is
@@ -243,7 +243,8 @@ inline size_t pass_bytes(const RJLayout& L, unsigned long long words)
 }
 // Histogram of range bins (see run_passes) of in[0], in[step], ...
 int hist_launch_range(pyg_ctx* ctx, const longlong2* in, int64_t n, int64_t step, int CB, int sub,
-                      const long long* csplit, const long long* fsplit, unsigned long long* hist);
+                      const long long* csplit, const long long* fsplit, unsigned long long* hist,
+                      long long* mm = nullptr);
 // One relation for rp_partition_sides.  In: in, n, allow_sample, the
 // splitters (range mode) and an optional event recorded after the
 // relation's passes.  Out: the layout (counts included), the pass buffers
@@ -301,18 +302,6 @@ struct RPAfter {
 // after (optional): work on the partitions that needs no host round trip.
 int rp_partition_sides(pyg_ctx* ctx, RPSide* sd, int ns, int FB, bool two, unsigned* flags, unsigned* hflags,
                        cudaEvent_t hist_done, bool share_key_frame = false, const RPAfter* after = nullptr);
-
-// Partitions one relation into 2^FB partitions (hash bits, or ranges when
-// csplit is set; two passes when `two`): histogram (sampled when allowed
-// and n >= 2^25), layout, passes, and an exact redo if a sampled region
-// overflowed.  On success the partitions are in (two ? *P2 : *P1) at
-// L.fstart with L.count tuples each; the caller frees *P1 and *P2.  flags:
-// two device words (bulk copy never landed, region overflow); hflags: two
-// pinned host words; both need 4 words (see rp_partition_sides).  hist_ms /
-// hist_tuples (optional): the histogram's time and the tuples it read.
-int rp_partition(pyg_ctx* ctx, const longlong2* in, int64_t n, int FB, bool two, bool allow_sample,
-                 const long long* csplit, const long long* fsplit, RJLayout& L, void** P1, void** P2,
-                 unsigned* flags, unsigned* hflags, float* hist_ms = nullptr, int64_t* hist_tuples = nullptr);
 
 // Hash of the radix operators: multiplication by 2^64 / golden ratio
 // (Fibonacci hashing) after three xor-shifts.  Bit j of the product depends
