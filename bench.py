@@ -507,9 +507,11 @@ def join_roofline(pyg, phase, nR, nS, step_ms, hbm, peak_kind, theta):
                 "launches": ph, "algorithm": int(phase[0].algorithm), "radix_bits": int(phase[0].radix_bits),
                 "histogram_ms": round(mean("histogram_ms"), 3) if radix else None,
                 "histogram_tuples": int(phase[0].histogram_tuples) if radix else None,
-                # Host round trips inside the step: the layouts formed from the
-                # histograms (before the build side's passes), and the work
-                # items formed from the partition counts (before the join).
+                # Beside the kernels: the layouts formed on the host from the
+                # histograms (before the build side's passes), and the probe
+                # phase outside the join kernel (the work items are formed on
+                # the device from the partition counts; the rest is its clears
+                # and the result's copy).
                 "host_layout_ms": round(mean("build_partition_ms") - mean2("build_pass_ms", 0)
                                         - mean2("build_pass_ms", 1), 3) if radix else None,
                 "host_items_ms": round(mean("probe_ms") - mean("join_kernel_ms"), 3) if radix else None,

@@ -5,17 +5,18 @@
 // for the 16-byte (int64 key, int64 payload) case, B200-first:
 //
 //   1. histogram  one read of each relation counts the top `fine_bits`
-//                 bits of rj_hash(key) in a shared-memory histogram per CTA;
-//                 the host turns the counts into exact partition offsets.
+//                 bits of rj_hash(key) (large relations: of a sample) in a
+//                 shared-memory histogram per CTA; the host turns the counts
+//                 into partition offsets or regions with slack.
 //   2. partition  one or two tile passes (coarse bits, then the remaining
-//                 bits inside each coarse partition).  A CTA groups a
-//                 2048-tuple tile by partition in shared memory and writes
-//                 each group as one contiguous run; exact offsets mean no
-//                 capacity slack and no overflow path.
+//                 bits inside each coarse partition).  A CTA groups a tile
+//                 by partition in shared memory and writes each group as
+//                 one contiguous run.
 //   3. join       a persistent kernel takes work items (a build partition,
 //                 or a chunk of it, and a chunk of the matching probe
-//                 partition) from a queue.  The CTA builds the partition's
-//                 table in 192 KB of shared memory, then streams the probe
+//                 partition) from a queue formed on the device.  The CTA
+//                 builds the partition's table in shared memory (96 KB, two
+//                 CTAs per SM, or 192 KB), then streams the probe
 //                 chunk from HBM against it.  No grid-wide barrier: CTAs
 //                 never wait for one another, and table lookups never leave
 //                 the SM.

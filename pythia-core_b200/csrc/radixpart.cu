@@ -182,14 +182,13 @@ struct RJPass {
     RJModel model;
 };
 
-// Element formats: a pass reads 16-byte tuples (the relation, or unpacked
-// intermediates) or packed 8-byte words, and writes either.  Packed input
-// tiles hold 4096 words (bins of at most 2^8, so the staged bin index is
-// one byte); 16-byte tiles hold 2048 tuples.  Both fit two CTAs per SM.
 // How a pass computes a tuple's bin, fixed per kernel instance so that no
 // per-tuple branch chooses it.
 enum RJMode { RJ_MODE_HASH = 0, RJ_MODE_MODEL = 1, RJ_MODE_RANGE = 2 };
 
+// Element formats: a pass reads 16-byte tuples (the relation, or unpacked
+// intermediates) or packed 8-byte words, and writes either.  Packed input
+// has bins of at most 2^8, so the staged bin index is one byte.
 template <bool IN8, bool OUT8, int MODE>
 struct RJFmt {
     using In = typename std::conditional<IN8, unsigned long long, longlong2>::type;
@@ -252,8 +251,8 @@ __device__ RJTileRange rj_tile_range(const RJPass& a, RJSegCursor& c, long long 
 //   packed in and out, hash          probe pass 2 4.03 ms.  256 bins: two
 //     control warps reserve four each per lane (one warp: 4.70 ms).
 //   model and range bins wait on their leaf and splitter loads and take
-//     whichever shape measured best: 3.00 and 1.77 ms (model), 3.92 and
-//     2.90 ms (range, unpacked), group-by 0.72 ms (hash, unpacked).
+//     whichever shape measured best: 2.87 and 2.20 ms (model), 3.71 and
+//     2.38 ms (range), group-by 0.72 ms (hash, unpacked).
 // Against one kernel shape of 2 x 256 or 512 threads without control warps,
 // three barriers per tile and reservations waited for inside a tile: 6.78,
 // 4.66, 3.09, 1.95, 3.92, 3.05 and 0.81 ms.
@@ -979,9 +978,8 @@ int rp_partition_sides(pyg_ctx* ctx, RPSide* sd, int ns, int FB, bool two, unsig
                        cudaEvent_t hist_done, bool share_key_frame, const RPAfter* after)
 {
     // Coarse bits of the first of two passes.  Unpacked layouts split FB
-    // evenly (2048-tuple tiles); packed layouts keep the second pass at 2^8
-    // bins, so that its 4096-word tiles use one-byte bin indexes and both
-    // passes write runs of about 16 words.  The unpacked split has at least
+    // evenly; packed layouts keep the second pass at 2^8 bins, so that its
+    // tiles use one-byte bin indexes and write runs of about 20 words.  The unpacked split has at least
     // as many coarse partitions, so its metadata size covers both.
     auto coarse_bits = [&](bool packed) { return !two ? FB : (packed ? std::max(1, FB - 8) : (FB + 1) / 2); };
     const int F = 1 << FB;

@@ -10,15 +10,15 @@ known workload:
 Inputs are sized to exceed the 126 MB L2 while staying a few GB on the
 device.  Cases and the kernels they launch:
 
-  radix      R 2^24 x S 2^27 PK-FK radix join      rj_hist, rj_partition, rj_join
+  radix      R 2^24 x S 2^27 PK-FK radix join      rj_hist, rj_partition, rj_items, rj_join32
   direct     R 2^20 x S 2^24 join, one HBM table    dj_clear, dj_build, dj_probe
   groupby16  2^26 (int64, int64), G = 16 / 1024 / 2^16   gbr_tiny / gbr_direct / gbr_part
   groupby-zipf  2^26 tuples, G = 2^16, Zipf(1.0) ids     rj_hist, rj_partition, gbr_part
-  composite  2^25 (int32, int32, int64), G = 2^16    groupby_kernel
+  composite  2^25 (int32, int32, int64), G = 2^16    rj_partition, gbr_part
   partition  2^25 tuples, exactrange, fan-out 64     pt_hist, pt_scatter
-  sort       2^24 tuples                            rs_hist, rs_scatter
+  sort       2^24 tuples                            os_range, os_hist, os_pass
   mpsm       R 2^22 x S 2^24, sampled or learned splitters   mp16 path (aggregate sink)
-  mpsm-mat   R 2^20 x S 2^22, materialised          mp_tile_sort, mp_merge, mp_join
+  mpsm-mat   R 2^20 x S 2^22, materialised          os_pass, mm_join
   cdf        2^21-key sample, 1024 leaves           cdf training kernels
   batch      64 fragments, builds 2^12..2^18        batch_kernel
 """
