@@ -34,6 +34,8 @@ namespace pyg {
 // A random hash at half load gives a warp of 32 x 4 lookups a longest chain of
 // about ten dependent reads; consecutive keys here hardly meet: build of 1 M
 // keys 67 -> 19 us, materialising probe of 8 M 163 -> 88 us (against mix64).
+// Random keys keep their chains: build, probe and sort of the joined rows take
+// 487 us with keys 1..n, 625 us with random 31- or 64-bit keys.
 __device__ __forceinline__ uint64_t ht_slot(uint64_t k, uint64_t cap)
 {
     const uint64_t h = rj_hash(k);
