@@ -561,7 +561,7 @@ __global__ void __launch_bounds__(RJShape<IN8, OUT8, MODE>::THREADS, RJShape<IN8
     }
     // ---- workers
     Out* out = reinterpret_cast<Out*>(a.out);
-    unsigned miss = 0;  // high halves of packed offsets: nonzero when a tuple was outside the frame
+    unsigned miss = 0;  // nonzero when a tuple was outside the packed frame
     __syncthreads();
     long long k = 0;
     for (long long tile = blockIdx.x;; tile += gridDim.x, ++k) {
@@ -590,10 +590,16 @@ __global__ void __launch_bounds__(RJShape<IN8, OUT8, MODE>::THREADS, RJShape<IN8
                     if constexpr (IN8 || !OUT8) {
                         t[j] = e;
                     } else {
-                        // Pack: (key - kbase) | (payload - pbase) << 32.
+                        // Pack: (key - kbase) | (payload - pbase) << 32.  The
+                        // key offset 2^32 - 1, which marks free slots in the
+                        // tables built from the words, is outside the frame
+                        // too: dk + 1 then carries into its high half (and dk
+                        // itself has one where dk + 1 wraps to 0).  A comparison
+                        // dk >= 2^32 - 1 measured 12872 us, this 12816, neither
+                        // test 12764 (R 2^27 x S 2^30).
                         const unsigned long long dk = (unsigned long long)e.x - a.kbase;
                         const unsigned long long dp = (unsigned long long)e.y - a.pbase;
-                        miss |= (unsigned)(dk >> 32) | (unsigned)(dp >> 32);
+                        miss |= (unsigned)(dk >> 32) | (unsigned)((dk + 1) >> 32) | (unsigned)(dp >> 32);
                         t[j] = (dk & 0xFFFFFFFFULL) | (dp << 32);
                     }
                     if constexpr (Smem::TABLES) {

@@ -170,7 +170,9 @@ void layout_sampled(const std::vector<unsigned long long>& sc, long long step, i
 // Frame of a packed layout from the key and payload ranges seen by the
 // histogram ([kmin, kmax], [pmin, pmax], signed).  exact: the ranges cover
 // every tuple; else they come from a sample and must leave a margin of at
-// least 2^30 on each side.  Offsets stay below 2^32 - 1.  key_base (when
+// least 2^30 on each side.  Key offsets stay below 2^32 - 1: an exact frame
+// ends there, and a pass reports a tuple that a sampled frame put there or
+// beyond as a frame miss.  key_base (when
 // given) is a key frame shared with another relation (common_key_frame).
 // Returns false when no frame fits.
 bool pack_frame(long long kmin, long long kmax, long long pmin, long long pmax, bool exact, RJLayout& L,
