@@ -10,7 +10,8 @@
  * wave's clear and build items before the probe items of the wave before
  * it).  A probe item waits (with a bounded spin that reports
  * PYG_ERR_TIMEOUT instead of hanging) only for build items of its own
- * fragment that other CTAs already dequeued.  The queue reset and the
+ * fragment (clear items, when its build side is empty) that other CTAs
+ * already dequeued.  The queue reset and the
  * kernel are captured once in a CUDA graph and replayed per run.
  *
  * Fragments whose build side has at least `large_build` tuples are not

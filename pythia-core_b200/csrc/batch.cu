@@ -127,8 +127,12 @@ __global__ void __launch_bounds__(1024) batch_kernel(BatchDev d)
         if (threadIdx.x < RES_WORDS) red[threadIdx.x] = 0;
         if (threadIdx.x == 0) {
             ok = 1;
-            if (w.kind == 1) ok = wait_count(&d.init_done[w.frag], (unsigned)f.n_init, d.st);
-            if (w.kind == 2) ok = wait_count(&d.build_done[w.frag], (unsigned)f.n_build, d.st);
+            // Build items wait for the table's clears, probe items for its
+            // builds, or for the clears where there is nothing to build.
+            if (w.kind == 1 || (w.kind == 2 && f.n_build == 0))
+                ok = wait_count(&d.init_done[w.frag], (unsigned)f.n_init, d.st);
+            else if (w.kind == 2)
+                ok = wait_count(&d.build_done[w.frag], (unsigned)f.n_build, d.st);
             __threadfence();
             dupf = w.kind == 2 ? (int)*(volatile unsigned*)&d.dup[w.frag] : 0;
         }
