@@ -74,6 +74,14 @@ void* pyg_ctx_stream(pyg_ctx* ctx);
 int pyg_ctx_sync(pyg_ctx* ctx);
 /* Number of kernels this context has launched so far. */
 int64_t pyg_ctx_kernel_launches(pyg_ctx* ctx);
+/* Failure-detection test hook: in the context's next radix sort, or
+ * materialising merge join, of more than one tile, the first tile keeps its
+ * counts to itself.  The bounded waits of the tiles behind it then give up
+ * (about two seconds), the call returns PYG_ERR_TIMEOUT and the context
+ * stays usable. */
+#define PYG_STALL_SORT   0
+#define PYG_STALL_MERGE  1
+int pyg_inject_stall(pyg_ctx* ctx, int32_t where);
 const char* pyg_last_error(void);
 const char* pyg_version(void);
 

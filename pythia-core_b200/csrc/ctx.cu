@@ -258,6 +258,18 @@ int pyg_ctx_sync(pyg_ctx* ctx)
     return PYG_OK;
 }
 
+int pyg_inject_stall(pyg_ctx* ctx, int32_t where)
+{
+    int rc = check_ctx(ctx);
+    if (rc) return rc;
+    if (where != PYG_STALL_SORT && where != PYG_STALL_MERGE) {
+        set_error("pyg_inject_stall: unknown place %d", where);
+        return PYG_ERR_ARG;
+    }
+    (where == PYG_STALL_SORT ? ctx->stall_sort : ctx->stall_merge) = 1;
+    return PYG_OK;
+}
+
 int64_t pyg_ctx_kernel_launches(pyg_ctx* ctx) { return ctx ? ctx->launches : 0; }
 
 int pyg_alloc(pyg_ctx* ctx, size_t bytes, void** out)

@@ -208,8 +208,10 @@ __global__ void gb_compact_kernel(const ulonglong4* __restrict__ table, uint64_t
 
 __global__ void gb_write_sorted_kernel(const ulonglong4* __restrict__ table, const ulonglong2* __restrict__ items,
                                        int64_t n, int64_t sentinel_pos, OutSpec o, uint64_t sent_key,
-                                       uint64_t sent_sum, uint64_t sent_cnt, uint8_t* out)
+                                       uint64_t sent_sum, uint64_t sent_cnt, uint8_t* out,
+                                       const unsigned* __restrict__ err)
 {
+    if (*err) return;  // the sort of the items gave up: slot numbers may be anything
     // Rows before sentinel_pos come from slot items[i].y, the sentinel group (if any)
     // sits at sentinel_pos, the rest shift by one.
     int64_t total = n + (sentinel_pos >= 0 ? 1 : 0);
@@ -441,7 +443,8 @@ extern "C" int pyg_groupby(pyg_ctx* ctx, const pyg_rel* in, const int32_t* key_c
         }
         if (!rc && total > 0) {
             gb_write_sorted_kernel<<<grid_for(ctx, total, threads, 4, 8), threads, 0, ctx->stream>>>(
-                table, sorted, g, sentinel_pos, o, kEmptyKey, sent_sum, sent_cnt, (uint8_t*)out);
+                table, sorted, g, sentinel_pos, o, kEmptyKey, sent_sum, sent_cnt, (uint8_t*)out,
+                (const unsigned*)(ctx->dcounters + SORT_ERR_WORD));
             PYG_LAUNCHED(ctx);
         }
         dfree(ctx, buf);

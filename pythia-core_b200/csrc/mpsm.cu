@@ -243,6 +243,7 @@ struct MatArgs {
     unsigned* ticket;     // zeroed, with status
     unsigned long long* status;
     unsigned* err;
+    int64_t mute;         // a tile that publishes nothing (test hook; else -1)
     unsigned long long* total;
     const uint8_t* rbase;  // original relations (row gather)
     const uint8_t* sbase;
@@ -291,10 +292,11 @@ __global__ void __launch_bounds__(MM_THREADS) mm_join_kernel(MatArgs a)
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     if (tid == 0) {
         ticket = atomicAdd(a.ticket, 1u);
-        ok = 1;
+        ok = *(volatile unsigned*)a.err == 0;
         many = 0;
     }
     __syncthreads();
+    if (!ok) return;  // a sort gave up: the items' row numbers may be anything
     const int64_t tile = ticket, s0 = tile * MM_TILE;
     const int n = a.nS - s0 < MM_TILE ? (int)(a.nS - s0) : MM_TILE;
     for (int i = tid; i < n; i += MM_THREADS) ss[i] = a.S[s0 + i];
@@ -418,7 +420,7 @@ __global__ void __launch_bounds__(MM_THREADS) mm_join_kernel(MatArgs a)
     // Rows before this tile.
     if (w == 0) {
         unsigned long long before = 0;
-        const bool found = lb_prefix(a.status, tile, all, a.err, before);
+        const bool found = tile == a.mute || lb_prefix(a.status, tile, all, a.err, before);
         if (lane == 0) {
             if (!found) ok = 0;
             base_s = before;
@@ -646,6 +648,8 @@ static int mpsm_materialize(pyg_ctx* ctx, const pyg_rel* build, const pyg_rel& R
     a.ticket = (unsigned*)(status + tiles);
     a.status = status;
     a.err = (unsigned*)(ctx->dcounters + SORT_ERR_WORD);
+    a.mute = ctx->stall_merge && tiles > 1 ? 0 : -1;
+    if (a.mute == 0) ctx->stall_merge = 0;
     a.total = ctx->dcounters + 112;
     a.rbase = (const uint8_t*)R.base;
     a.sbase = (const uint8_t*)S.base;

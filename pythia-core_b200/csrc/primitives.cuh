@@ -14,7 +14,8 @@ int exclusive_scan_u64(pyg_ctx* ctx, const unsigned long long* in, unsigned long
 // `field` (0 or 1), and of bare 64-bit keys.  Each reads the key range back
 // (one stream synchronisation) beyond 4096 elements.  After the caller's
 // next synchronisation of the stream, sort_status reports a pass whose
-// bounded device-side wait gave up.
+// bounded device-side wait gave up; the result is then undefined, and a
+// kernel that takes row numbers from it must look at the error word first.
 //
 // Into out (may not alias in).
 int radix_sort16_to(pyg_ctx* ctx, const ulonglong2* in, ulonglong2* out, int64_t n, int field, bool is_signed);
@@ -58,7 +59,8 @@ constexpr int64_t CDF_MPSM_SAMPLE = (int64_t)1 << 21;
 int estimate_distinct_keys(pyg_ctx* ctx, const uint8_t* base, int64_t n, int32_t tb, const KeySpec& ks,
                            int64_t* out);
 
-// Gather rows: out[i] = in[items[i].y] for tuples of tb bytes.
+// Gather rows: out[i] = in[items[i].y] for tuples of tb bytes.  Nothing is
+// read when the sort of the items gave up.
 int gather_rows(pyg_ctx* ctx, const uint8_t* in, const ulonglong2* items, int64_t n, int32_t tb, uint8_t* out);
 
 }  // namespace pyg

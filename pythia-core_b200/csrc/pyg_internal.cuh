@@ -36,6 +36,9 @@ struct pyg_ctx {
     // Bump cursor into the pinned upload area (after the scalar and stage
     // areas) used by stage_h2d.
     size_t up_cursor;
+    // Test hooks (pyg_inject_stall): the next sort pass, or merge, whose
+    // first tile publishes nothing.
+    int stall_sort, stall_merge;
 };
 
 namespace pyg {

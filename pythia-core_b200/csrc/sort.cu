@@ -343,7 +343,7 @@ template <typename Item, int FIELD>
 __global__ void __launch_bounds__(OsShape<Item>::THREADS, OsShape<Item>::MINB)
     os_pass_kernel(const Item* __restrict__ in, Item* __restrict__ out, int64_t n, uint64_t base, int pass,
                    OsScratch* __restrict__ sc, unsigned long long* __restrict__ status,
-                   unsigned* __restrict__ err)
+                   unsigned* __restrict__ err, int64_t mute)
 {
     using S = OsShape<Item>;
     constexpr int PER = S::PER, TILE = S::TILE, WARPS = S::WARPS;
@@ -359,10 +359,13 @@ __global__ void __launch_bounds__(OsShape<Item>::THREADS, OsShape<Item>::MINB)
     const unsigned agg_tag = 2u * (unsigned)pass + 1u;
     if (tid == 0) {
         ticket = atomicAdd(&sc->ticket[pass], 1u);
-        ok = 1;
+        ok = *(volatile unsigned*)err == 0;
     }
     for (int b = tid; b < WARPS * OS_BINS; b += S::THREADS) (&wcnt[0][0])[b] = 0;
     __syncthreads();
+    // A pass that gave up left tiles unwritten: what is read here is then no
+    // permutation of what was counted, and its digits have no bound.
+    if (!ok) return;
     const int64_t tile = ticket;
     const int64_t first = tile * TILE;
     const int count = n - first < TILE ? (int)(n - first) : TILE;
@@ -408,7 +411,7 @@ __global__ void __launch_bounds__(OsShape<Item>::THREADS, OsShape<Item>::MINB)
     if (tid < OS_BINS) {
         for (int v = 0; v < WARPS; ++v) c += wcnt[v][tid];
         const unsigned real = tid == OS_BINS - 1 ? c - (unsigned)(TILE - count) : c;
-        lb_store(st + tid, ((unsigned long long)real << 8) | (tile == 0 ? agg_tag + 1 : agg_tag));
+        if (tile != mute) lb_store(st + tid, ((unsigned long long)real << 8) | (tile == 0 ? agg_tag + 1 : agg_tag));
         incl = c;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -439,9 +442,11 @@ __global__ void __launch_bounds__(OsShape<Item>::THREADS, OsShape<Item>::MINB)
     if (tid < OS_BINS) {
         unsigned long long before = 0;
         if (tile > 0) {
-            if (!os_look_back(status, tile, tid, agg_tag, err, before)) ok = 0;
             const unsigned real = tid == OS_BINS - 1 ? c - (unsigned)(TILE - count) : c;
-            lb_store(st + tid, ((before + real) << 8) | (agg_tag + 1));
+            if (os_look_back(status, tile, tid, agg_tag, err, before))
+                lb_store(st + tid, ((before + real) << 8) | (agg_tag + 1));
+            else
+                ok = 0;
         }
         gbase[tid] = sc->hist[pass][tid] + before - start;
     }
@@ -568,10 +573,13 @@ static int os_passes(pyg_ctx* ctx, const Item* in, Item* dst0, Item* dst1, int64
         auto kern = os_pass_kernel<Item, FIELD>;
         PYG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM));
         const Item* src = in;
-        for (int p = 0; p < plan.passes; ++p) {
+        int64_t mute = ctx->stall_sort && tiles > 1 ? 0 : -1;
+        if (mute == 0) ctx->stall_sort = 0;
+        for (int p = 0; p < plan.passes; ++p, mute = -1) {
             Item* dst = p & 1 ? dst1 : dst0;
             kern<<<(unsigned)tiles, S::THREADS, S::SMEM, ctx->stream>>>(src, dst, n, plan.base, p, sc, status,
-                                                                  (unsigned*)(ctx->dcounters + SORT_ERR_WORD));
+                                                                        (unsigned*)(ctx->dcounters + SORT_ERR_WORD),
+                                                                        mute);
             PYG_LAUNCHED(ctx);
             src = dst;
         }
@@ -684,10 +692,13 @@ int radix_sort16_swap(pyg_ctx* ctx, ulonglong2* a, ulonglong2* b, int64_t n, int
 // ---------------------------------------------------------------------------
 // Gather, key extraction, sort entry point.
 
+// err: the error word of the sort that ordered the items (row numbers of a
+// sort that gave up may be anything).
 template <typename V>
 __global__ void gather_kernel(const V* __restrict__ in, const ulonglong2* __restrict__ items, int64_t n, int words,
-                              V* __restrict__ out)
+                              V* __restrict__ out, const unsigned* __restrict__ err)
 {
+    if (*err) return;
     int64_t total = n * words;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
         int64_t r = t / words;
@@ -699,19 +710,20 @@ __global__ void gather_kernel(const V* __restrict__ in, const ulonglong2* __rest
 int gather_rows(pyg_ctx* ctx, const uint8_t* in, const ulonglong2* items, int64_t n, int32_t tb, uint8_t* out)
 {
     if (n <= 0) return PYG_OK;
+    const unsigned* err = (const unsigned*)(ctx->dcounters + SORT_ERR_WORD);
     int threads = 256;
     if (tb % 16 == 0 && (uintptr_t)in % 16 == 0 && (uintptr_t)out % 16 == 0) {
         gather_kernel<uint4><<<grid_for(ctx, n * (tb / 16), threads, 4, 8), threads, 0, ctx->stream>>>(
-            (const uint4*)in, items, n, tb / 16, (uint4*)out);
+            (const uint4*)in, items, n, tb / 16, (uint4*)out, err);
     } else if (tb % 8 == 0 && (uintptr_t)in % 8 == 0 && (uintptr_t)out % 8 == 0) {
         gather_kernel<uint2><<<grid_for(ctx, n * (tb / 8), threads, 4, 8), threads, 0, ctx->stream>>>(
-            (const uint2*)in, items, n, tb / 8, (uint2*)out);
+            (const uint2*)in, items, n, tb / 8, (uint2*)out, err);
     } else if (tb % 4 == 0 && (uintptr_t)in % 4 == 0 && (uintptr_t)out % 4 == 0) {
         gather_kernel<unsigned><<<grid_for(ctx, n * (tb / 4), threads, 4, 8), threads, 0, ctx->stream>>>(
-            (const unsigned*)in, items, n, tb / 4, (unsigned*)out);
+            (const unsigned*)in, items, n, tb / 4, (unsigned*)out, err);
     } else {
         gather_kernel<unsigned char><<<grid_for(ctx, n * tb, threads, 4, 8), threads, 0, ctx->stream>>>(
-            in, items, n, tb, out);
+            in, items, n, tb, out, err);
     }
     PYG_LAUNCHED(ctx);
     return PYG_OK;

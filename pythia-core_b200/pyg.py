@@ -154,6 +154,7 @@ SIGNATURES = [
     ("pyg_hashjoin_agg_noalloc", C.c_int, [_P, _I64, _P, _I64, _P, _P]),
     ("pyg_groupby", C.c_int, [_P, C.POINTER(pyg_rel), _PI32, _I32, _I32, _I32, _I32, _I64, _P, _I64, _PI64]),
     ("pyg_partition", C.c_int, [_P, C.POINTER(pyg_rel), _I32, C.POINTER(pyg_splitter), _P, _PI64]),
+    ("pyg_inject_stall", C.c_int, [_P, _I32]),
     ("pyg_sort", C.c_int, [_P, C.POINTER(pyg_rel), _I32, _P]),
     ("pyg_lower_bound", C.c_int, [_P, C.POINTER(pyg_rel), _I32, _P, _I64, _P]),
     ("pyg_sortlimit", C.c_int, [_P, C.POINTER(pyg_rel), _PI32, _I32, _I32, _I64, _P, _I64, _PI64]),
