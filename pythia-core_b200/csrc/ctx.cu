@@ -87,6 +87,7 @@ int dalloc(pyg_ctx* ctx, void** p, size_t bytes)
     cudaError_t e = cudaMallocAsync(p, bytes, ctx->stream);
     if (e != cudaSuccess) {
         *p = nullptr;
+        cudaGetLastError();  // reported here: the next launch's check must not find it again
         return cuda_status(e, "cudaMallocAsync");
     }
     return PYG_OK;

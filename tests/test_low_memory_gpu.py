@@ -1,0 +1,52 @@
+"""Little device memory: a call that cannot run reports PYG_ERR_OOM once.  Each case runs in a process of its own that first takes
+all device memory but a stated rest."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+HEAD = """
+import sys
+sys.path.insert(0, sys.argv[1] + "/pythia-core_b200")
+import torch, pyg
+I32, I64 = pyg.INT32, pyg.INT64
+ctx = pyg.Ctx(0)
+def leave(mib):
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    free, _ = torch.cuda.mem_get_info()
+    return torch.empty(free - (mib << 20), dtype=torch.uint8, device="cuda")
+def small_join():  # loads the kernels and proves the context
+    k = torch.arange(10000, device="cuda")
+    R = torch.stack([k, k], 1).contiguous()
+    for algo in (pyg.JOIN_DIRECT, pyg.JOIN_RADIX):
+        n, _ = ctx.hashjoin_agg(pyg.Rel(R, 10000, [I64, I64]), [0], pyg.Rel(R, 10000, [I64, I64]), [0], [(0, 1), (1, 1)],
+                                algo)
+        assert n == 10000
+small_join()
+"""
+
+# Two buffers of 2 GiB do not fit: an error, after which the context works.
+SORT = HEAD + """
+n = 1 << 27
+A = torch.randint(-(1 << 62), 1 << 62, (n, 2), device="cuda")
+out = torch.empty_like(A)
+hog = leave(1000)
+try:
+    ctx.sort(pyg.Rel(A, n, [I64, I64]), 0, out)
+    raise SystemExit("the sort was expected to run out of memory")
+except pyg.PygError as e:
+    assert e.code == pyg.PYG_ERR_OOM, e.code
+small_join()
+"""
+
+
+@pytest.mark.parametrize("script", [SORT], ids=["sort"])
+def test_little_memory(torch_cuda, script):
+    torch_cuda.cuda.empty_cache()
+    r = subprocess.run([sys.executable, "-c", script, ROOT], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
