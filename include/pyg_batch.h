@@ -15,8 +15,8 @@
  * kernel are captured once in a CUDA graph and replayed per run.
  *
  * Fragments whose build side has at least `large_build` tuples are not
- * queued: their tables would not stay in L2, so after the graph they run one by one
- * with the algorithm pyg_hashjoin_agg would pick.  Those that take the
+ * queued: their tables would not stay in L2, so after the graph they run one
+ * by one with the algorithm pyg_hashjoin_agg would pick.  Those that take the
  * direct join are enqueued back to back with no host synchronisation
  * between them (their counters stay on the device until the run's single
  * synchronisation; a build side with a repeated key is answered by the
@@ -51,8 +51,9 @@ typedef struct pyg_tuning {
     float load_factor;           /* per-fragment table load factor           */
     int32_t chunk_tuples;        /* work-item grain in tuples                */
     int32_t large_build;         /* build tuples from which a fragment runs
-                                    as its own join (0: 2^21, and those
-                                    beyond 1.3 GB of queued tables)       */
+                                    as its own join.  0: 2^21, and those
+                                    beyond 1.3 GB of queued tables (2^16
+                                    when that memory cannot be had)       */
 } pyg_tuning;
 
 /* Plans n fragments (tuning NULL: the autotuner's cached choice, else

@@ -59,9 +59,9 @@ constexpr long long kWaitLimit = 1LL << 22;  // x ~256 ns sleeps, about one seco
 // their own calls, 2101 us from 2^18, 1948 us from 2^21 (keys 1..n; random
 // 31-bit keys: 4.76 ms, where 2^16 and one fragment after another took 5.23).
 constexpr int64_t kLargeBuild = (int64_t)1 << 21;
-// By default at most this many table slots (20 bytes each) are queued, the
-// smallest fragments first; the others run as their own joins, whose table
-// is one buffer that they share.
+// Unless the caller states a threshold, at most this many table slots (20
+// bytes each) are queued, the smallest build sides first; the others run as
+// their own joins, whose table is one buffer that they share.
 constexpr uint64_t kQueueSlots = (uint64_t)1 << 26;
 // The threshold when even that much memory cannot be had.
 constexpr int64_t kLargeBuildLowMem = (int64_t)1 << 16;
@@ -413,34 +413,48 @@ int pyg_batch_create(pyg_ctx* ctx, const pyg_fragment* frags, int32_t n, const p
     pyg_batch* b = new pyg_batch();
     b->n = n;
     b->tuning = t;
-    const int64_t large_build = t.large_build > 0 ? t.large_build : kLargeBuild;
-    std::vector<char> is_large(n, 0);
-    for (int i = 0; i < n; ++i)
-        if (frags[i].nbuild >= large_build) {
-            is_large[i] = 1;
-            b->large.push_back(i);
-            b->large_frag.push_back(frags[i]);
-        }
-    if (!b->large.empty()) {
-        int rc = batch_alloc(ctx, b, (void**)&b->large_words, b->large.size() * 16 * sizeof(unsigned long long));
-        if (rc) {
-            pyg_batch_free(ctx, b);
-            return rc;
-        }
-    }
-    // Tables: one arena of 16-byte slots and one of extra-copy counters,
-    // per-fragment capacity nbuild / load factor (queued fragments only).
+    // Fragments of `threshold` build tuples and more run as their own joins;
+    // where the threshold is not the caller's, so do those past the first
+    // kQueueSlots table slots, counted from the smallest build.
+    const bool automatic = !tuning || t.large_build == 0;
     std::vector<FragDesc> fd(n);
-    uint64_t total_slots = 0;
-    for (int i = 0; i < n; ++i) {
-        uint64_t cap = is_large[i] ? 0 : (uint64_t)((double)frags[i].nbuild / t.load_factor) + 64;
-        fd[i].cap = cap;
-        total_slots += cap;
-    }
+    std::vector<char> is_large(n);
+    std::vector<int32_t> by_build(n);
+    for (int i = 0; i < n; ++i) by_build[i] = i;
+    std::stable_sort(by_build.begin(), by_build.end(),
+                     [&](int a, int c) { return frags[a].nbuild < frags[c].nbuild; });
     ulonglong2* arena;
     unsigned* extra;
-    if ((rc = batch_alloc(ctx, b, (void**)&arena, std::max<uint64_t>(total_slots, 1) * sizeof(ulonglong2))) ||
-        (rc = batch_alloc(ctx, b, (void**)&extra, std::max<uint64_t>(total_slots, 1) * sizeof(unsigned)))) {
+    // Tables: one arena of 16-byte slots and one of extra-copy counters,
+    // per-fragment capacity nbuild / load factor (queued fragments only).
+    auto plan_tables = [&](int64_t threshold) -> int {
+        for (void* p : b->bufs) dfree(ctx, p);
+        b->bufs.clear();
+        b->large.clear();
+        b->large_frag.clear();
+        uint64_t total_slots = 0;
+        for (int i : by_build) {
+            const uint64_t cap = (uint64_t)((double)frags[i].nbuild / t.load_factor) + 64;
+            is_large[i] = frags[i].nbuild >= threshold || (automatic && total_slots + cap > kQueueSlots);
+            fd[i].cap = is_large[i] ? 0 : cap;
+            total_slots += fd[i].cap;
+        }
+        for (int i = 0; i < n; ++i)
+            if (is_large[i]) {
+                b->large.push_back(i);
+                b->large_frag.push_back(frags[i]);
+            }
+        int r = PYG_OK;
+        if (!b->large.empty())
+            r = batch_alloc(ctx, b, (void**)&b->large_words, b->large.size() * 16 * sizeof(unsigned long long));
+        if (!r) r = batch_alloc(ctx, b, (void**)&arena, std::max<uint64_t>(total_slots, 1) * sizeof(ulonglong2));
+        if (!r) r = batch_alloc(ctx, b, (void**)&extra, std::max<uint64_t>(total_slots, 1) * sizeof(unsigned));
+        return r;
+    };
+    const int64_t large_build = t.large_build > 0 ? t.large_build : kLargeBuild;
+    rc = plan_tables(large_build);
+    if (rc == PYG_ERR_OOM && automatic && large_build > kLargeBuildLowMem) rc = plan_tables(kLargeBuildLowMem);
+    if (rc) {
         pyg_batch_free(ctx, b);
         return rc;
     }

@@ -1,4 +1,6 @@
-"""Little device memory: a call that cannot run reports PYG_ERR_OOM once.  Each case runs in a process of its own that first takes
+"""Calls whose faster route needs more device memory than there is fall back
+to the one that needs less, and a call that cannot run at all reports
+PYG_ERR_OOM once.  Each case runs in a process of its own that first takes
 all device memory but a stated rest."""
 import os
 import subprocess
@@ -30,6 +32,24 @@ def small_join():  # loads the kernels and proves the context
 small_join()
 """
 
+# 24 fragments whose tables would take 1.1 GiB together.
+BATCH = HEAD + """
+pairs = []
+for i in range(24):
+    nb = 1200000 + i
+    k = torch.randperm(nb, device="cuda")
+    R = torch.stack([k, k], 1).contiguous()
+    pairs.append((R, nb, R[: 5000 + i].clone(), 5000 + i))
+want = [(n, 2 * int(S[:, 0].sum())) for _, _, S, n in pairs]
+hog = leave(700)
+b = ctx.batch_create(ctx.fragments(pairs))
+for _ in range(2):
+    rc, c, s, _ = ctx.batch_run(b, len(pairs))
+    assert rc == 0 and [(int(x), int(y)) for x, y in zip(c, s)] == want
+ctx.batch_free(b)
+small_join()
+"""
+
 # Two buffers of 2 GiB do not fit: an error, after which the context works.
 SORT = HEAD + """
 n = 1 << 27
@@ -45,7 +65,7 @@ small_join()
 """
 
 
-@pytest.mark.parametrize("script", [SORT], ids=["sort"])
+@pytest.mark.parametrize("script", [BATCH, SORT], ids=["batch", "sort"])
 def test_little_memory(torch_cuda, script):
     torch_cuda.cuda.empty_cache()
     r = subprocess.run([sys.executable, "-c", script, ROOT], capture_output=True, text=True, timeout=300)
