@@ -283,7 +283,7 @@ int pyg_partition(pyg_ctx* ctx, const pyg_rel* in, int32_t key_col, const pyg_sp
 /* ---- sort ----------------------------------------------------------- */
 /* Replaces SortOp / TupleBuffer::sort<KeyT> (operators/sort.cpp:87-311,
  * util/buffer.inl:119-452): orders tuples by the signed key column.
- * Stable.  out may not alias in. */
+ * Stable.  out may be in's own buffer (a copy of it is sorted then). */
 int pyg_sort(pyg_ctx* ctx, const pyg_rel* in, int32_t key_col, void* out);
 
 /* Replaces SortLimit (operators/sortlimit.cpp:32-262, plan node

@@ -745,6 +745,20 @@ int sort_relation(pyg_ctx* ctx, const pyg_rel* r, int32_t key_col, void* out)
 {
     int64_t n = r->ntuples;
     if (n == 0) return PYG_OK;
+    const size_t bytes = (size_t)n * r->tuple_bytes;
+    if ((uintptr_t)out < (uintptr_t)r->base + bytes && (uintptr_t)r->base < (uintptr_t)out + bytes) {
+        // In place: the first pass (or the gather) would write tuples that
+        // others have yet to read, so a copy is sorted.
+        pyg_rel copy = *r;
+        void* buf;
+        int rc = dalloc(ctx, &buf, bytes);
+        if (rc) return rc;
+        copy.base = buf;
+        cudaError_t e = cudaMemcpyAsync(buf, r->base, bytes, cudaMemcpyDeviceToDevice, ctx->stream);
+        rc = e == cudaSuccess ? sort_relation(ctx, &copy, key_col, out) : cuda_status(e, "in-place sort");
+        dfree(ctx, buf);
+        return rc;
+    }
     int32_t off = r->col_offset[key_col], type = r->col_type[key_col];
     if (r->tuple_bytes == 16 && type == PYG_INT64 && (off == 0 || off == 8) && (uintptr_t)r->base % 16 == 0 &&
         (uintptr_t)out % 16 == 0)
