@@ -1049,6 +1049,15 @@ int rp_partition_sides(pyg_ctx* ctx, RPSide* sd, int ns, int FB, bool two, unsig
         if (sd[s].done) cudaEventRecord(sd[s].done, ctx->stream);
         return PYG_OK;
     };
+    // Relation s's layout from an exact histogram (one host round trip).
+    auto form_exact = [&](int s) -> int {
+        int r = hist_of(s, 1);
+        if (r) return r;
+        PYG_CUDA(cudaMemcpyAsync(hh_at(s), hist_at(s), (size_t)(F + 4) * 8, cudaMemcpyDeviceToHost, ctx->stream));
+        PYG_CUDA(cudaStreamSynchronize(ctx->stream));
+        form(s, hh_at(s), 1, true, nullptr);
+        return PYG_OK;
+    };
     do {
         if ((rc = dalloc(ctx, (void**)&meta, per * 8 * ns))) break;
         PYG_CUDA(cudaMemsetAsync(flags, 0, (size_t)16 * ns, ctx->stream));
@@ -1077,6 +1086,9 @@ int rp_partition_sides(pyg_ctx* ctx, RPSide* sd, int ns, int FB, bool two, unsig
         for (int s = 0; s < ns && !rc; ++s) {
             form(s, hh_at(s), step[s], !sample[s], common ? &ckb : nullptr);
             rc = launch(s);
+            // Not enough memory for a sampled layout's slack (a fifth of the
+            // relation with about 2^9 samples per partition): exact regions.
+            if (rc == PYG_ERR_OOM && sd[s].L.sampled && !(rc = form_exact(s))) rc = launch(s);
         }
         if (rc) break;
         PYG_CUDA(cudaMemcpyAsync(hflags, flags, (size_t)16 * ns, cudaMemcpyDeviceToHost, ctx->stream));
@@ -1114,10 +1126,7 @@ int rp_partition_sides(pyg_ctx* ctx, RPSide* sd, int ns, int FB, bool two, unsig
             // regions cannot overflow, and an exact frame misses nothing).
             sd[s].overflowed = true;
             sd[s].done = sd[s].begin = sd[s].mid = nullptr;  // the redo's time is not attributed to the relation
-            if ((rc = hist_of(s, 1))) break;
-            PYG_CUDA(cudaMemcpyAsync(hh_at(s), hist_at(s), (size_t)(F + 4) * 8, cudaMemcpyDeviceToHost, ctx->stream));
-            PYG_CUDA(cudaStreamSynchronize(ctx->stream));
-            form(s, hh_at(s), 1, true, nullptr);
+            if ((rc = form_exact(s))) break;
             PYG_CUDA(cudaMemsetAsync(flags + 4 * s, 0, 16, ctx->stream));
             if ((rc = launch(s))) break;
             PYG_CUDA(cudaMemcpyAsync(hflags + 4 * s, flags + 4 * s, 16, cudaMemcpyDeviceToHost, ctx->stream));

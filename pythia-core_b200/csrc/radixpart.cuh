@@ -295,7 +295,9 @@ struct RPAfter {
 // host round trip, both relations' passes (the second relation's layout is
 // formed while the first one's passes run), one more round trip for the
 // counts and flags, and an exact redo of a relation whose sampled region
-// overflowed or whose packed frame missed a tuple (the redo is unpacked).
+// overflowed or whose packed frame missed a tuple (the redo is packed again
+// where the exact ranges fit a frame).  A sampled layout whose slack does not
+// fit in device memory is replaced by an exact one.
 // flags: 4 device words per relation (bulk copy never landed, region
 // overflow, frame miss, unused); hflags: as many pinned host words.
 // hist_done (optional) is recorded after the histograms.

@@ -32,6 +32,24 @@ def small_join():  # loads the kernels and proves the context
 small_join()
 """
 
+# One sampled pass over 2^28 wide tuples: 4.0 GiB of exact regions, 4.8 GiB
+# with a sample's slack.
+JOIN = HEAD + """
+n, m = 1 << 28, 5000
+S = torch.empty(n, 2, dtype=torch.int64, device="cuda")
+S[:, 0] = torch.randint(0, m, (n,), device="cuda")
+S[:, 1] = 1
+S[::1000, 1] = 1 << 40
+sums = [int(S[:, 0].sum()) * 7, int(S[:, 1].sum())]
+k = torch.arange(m, device="cuda")
+R = torch.stack([k, k * 7], 1).contiguous()
+hog = leave(4500)
+got, s = ctx.hashjoin_agg(pyg.Rel(R, m, [I64, I64]), [0], pyg.Rel(S, n, [I64, I64]), [0], [(0, 1), (1, 1)],
+                          pyg.JOIN_RADIX, 7)
+assert got == n and [int(x) for x in s] == sums
+small_join()
+"""
+
 # 24 fragments whose tables would take 1.1 GiB together.
 BATCH = HEAD + """
 pairs = []
@@ -65,7 +83,7 @@ small_join()
 """
 
 
-@pytest.mark.parametrize("script", [BATCH, SORT], ids=["batch", "sort"])
+@pytest.mark.parametrize("script", [JOIN, BATCH, SORT], ids=["join", "batch", "sort"])
 def test_little_memory(torch_cuda, script):
     torch_cuda.cuda.empty_cache()
     r = subprocess.run([sys.executable, "-c", script, ROOT], capture_output=True, text=True, timeout=300)
