@@ -345,7 +345,7 @@ extern "C" int pyg_groupby(pyg_ctx* ctx, const pyg_rel* in, const int32_t* key_c
     // aggregated in shared memory (gbradix.cu).  The pair used to take the
     // generic kernel: 40 M tuples, 2^16 groups, 3.44 ms.
     const bool pair32 = ks.nkeys == 2 && ks.off0 == 0 && ks.off1 == 4;
-    const bool fast16 = a.tb == 16 && (pair32 || (ks.nkeys == 1 && ks.off0 == 0 && ks.type0 == PYG_INT64)) &&
+    bool fast16 = a.tb == 16 && (pair32 || (ks.nkeys == 1 && ks.off0 == 0 && ks.type0 == PYG_INT64)) &&
                         (!want_sum || (a.sum_off == 8 && a.sum_type == PYG_INT64)) && (uintptr_t)a.base % 16 == 0 &&
                         groupby16_eligible(expected_groups);
     ulonglong4* table = nullptr;
@@ -358,8 +358,14 @@ extern "C" int pyg_groupby(pyg_ctx* ctx, const pyg_rel* in, const int32_t* key_c
         a.table = table;
         a.cap = cap;
         if (a.n > 0 && fast16) {
-            if ((rc = groupby16_fill(ctx, a.base, a.n, pair32, want_sum, expected_groups, table, cap, a.flags))) break;
-        } else if (a.n > 0) {
+            rc = groupby16_fill(ctx, a.base, a.n, pair32, want_sum, expected_groups, table, cap, a.flags);
+            // No memory for the partitions (nothing was folded yet): the
+            // generic kernel needs none.
+            fast16 = rc != PYG_ERR_OOM;
+            if (!fast16) rc = PYG_OK;
+            if (rc) break;
+        }
+        if (a.n > 0 && !fast16) {
             int grid = grid_for(ctx, a.n, threads, 16, use_smem ? 2 : 8);
             if (use_smem) groupby_kernel<true><<<grid, threads, smem, ctx->stream>>>(a);
             else groupby_kernel<false><<<grid, threads, 0, ctx->stream>>>(a);
@@ -384,6 +390,7 @@ extern "C" int pyg_groupby(pyg_ctx* ctx, const pyg_rel* in, const int32_t* key_c
         cap *= 2;
     }
     if (rc) {
+        dfree(ctx, table);
         R.release(ctx);
         return rc;
     }

@@ -50,6 +50,27 @@ assert got == n and [int(x) for x in s] == sums
 small_join()
 """
 
+# (int32, int32) keys: no room for partitions of the 4 GiB input.
+GROUPBY = HEAD + """
+n, g = 1 << 28, 5000
+A = torch.empty(n, 2, dtype=torch.int64, device="cuda")
+ids = torch.randint(0, g, (n,), dtype=torch.int32, device="cuda")
+P = A.view(torch.int32).view(n, 4)
+P[:, 0] = ids
+P[:, 1] = 3
+A[:, 1] = 2
+cnt = torch.bincount(ids, minlength=g).cpu()
+del ids
+out = torch.empty(g, 3, dtype=torch.int64, device="cuda")
+hog = leave(1200)
+rc, got = ctx.groupby(pyg.Rel(A, n, [I32, I32, I64]), [0, 1], 3, 2, True, g, out, g)
+assert rc == 0 and got == g
+out = out.cpu()
+assert torch.equal(out[:, 0], torch.arange(g) | (3 << 32))
+assert torch.equal(out[:, 2], cnt) and torch.equal(out[:, 1], cnt * 2)
+small_join()
+"""
+
 # 24 fragments whose tables would take 1.1 GiB together.
 BATCH = HEAD + """
 pairs = []
@@ -83,7 +104,7 @@ small_join()
 """
 
 
-@pytest.mark.parametrize("script", [JOIN, BATCH, SORT], ids=["join", "batch", "sort"])
+@pytest.mark.parametrize("script", [JOIN, GROUPBY, BATCH, SORT], ids=["join", "groupby", "batch", "sort"])
 def test_little_memory(torch_cuda, script):
     torch_cuda.cuda.empty_cache()
     r = subprocess.run([sys.executable, "-c", script, ROOT], capture_output=True, text=True, timeout=300)
