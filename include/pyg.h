@@ -172,7 +172,10 @@ int pyg_hashjoin_probe_materialize(pyg_ctx* ctx, const pyg_hashtable* ht, const 
  * getNext, operators/join.cpp:548-757, feeding GenericAggregate).
  * PYG_JOIN_DIRECT: one table in HBM, probed in input order; for 16-byte
  * device relations a three-launch call with one host synchronisation whose
- * table lives in a buffer the context keeps between calls.
+ * table lives in a buffer the context keeps between calls; build sides of at
+ * most 6144 tuples take a single launch with tables in shared memory, sized
+ * without regard to load_factor, unless stats asks for the phases (which
+ * then are those of the three launches).
  * PYG_JOIN_RADIX: both sides partitioned by the top radix_bits bits of the
  * key hash first, then joined partition by partition with shared-memory
  * tables (16-byte (int64, int64) device relations, projection over

@@ -1056,7 +1056,9 @@ static int direct_join16(pyg_ctx* ctx, const longlong2* R, int64_t nR, const lon
                          unsigned long long res[3], bool* fallback, PhaseTimer* tm)
 {
     unsigned long long* h = (unsigned long long*)ctx->pinned;
-    if (nR <= SJ_MAX_BUILD && !tm->on) {  // phase times need the three launches
+    // Phase times need the three launches.  Load factors that no table
+    // accepts keep to them too, where one that leaves no room is refused.
+    if (nR <= SJ_MAX_BUILD && !tm->on && lf <= 0.95f) {
         int bits = 8;
         while (bits < SJ_MAX_BITS && ((int64_t)1 << bits) < 2 * nR) ++bits;
         PYG_CUDA(cudaFuncSetAttribute(sj_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 16 << SJ_MAX_BITS));
