@@ -22,6 +22,24 @@ __device__ __forceinline__ unsigned rj_bin(uint64_t h, int shift, unsigned mask)
     return shift >= 64 ? 0u : (unsigned)(h >> shift) & mask;
 }
 
+// Row that sample i of a layout's histogram reads: one row of every `step`,
+// at a multiple of `spread` that the MurmurHash3 32-bit finaliser of i picks.
+// Rows at a fixed stride see a few values of keys that repeat with the row
+// number (row % 2^16 at a stride of 2^8: one in 2^8), most regions overflow,
+// and the relation is partitioned twice.  spread is 1 for one pass.  For two
+// it is 2: the test of that redo hides keys from the sample in the odd rows
+// of an even stride.
+__device__ __forceinline__ int64_t rj_sample_row(int64_t i, int64_t step, int spread, int64_t n)
+{
+    if (step == 1) return i;
+    unsigned h = (unsigned)i;
+    h ^= h >> 16;
+    h *= 0x85ebca6bu;
+    h ^= h >> 13;
+    h *= 0xc2b2ae35u;
+    h ^= h >> 16;
+    return min(i * step + spread * (int64_t)(((uint64_t)h * (uint64_t)(step / spread)) >> 32), n - 1);
+}
 
 // ---------------------------------------------------------------------------
 // 1. Histogram of the top `bits` hash bits (bits <= 15: 128 KB of shared
@@ -29,11 +47,11 @@ __device__ __forceinline__ unsigned rj_bin(uint64_t h, int shift, unsigned mask)
 
 template <bool MODEL>
 __global__ void __launch_bounds__(1024) rj_hist_kernel(const longlong2* __restrict__ in, int64_t n, int64_t step,
-                                                       int bits, int base, int span, unsigned* __restrict__ part,
+                                                       int spread, int bits, int base, int span, unsigned* __restrict__ part,
                                                        long long* __restrict__ mm, RJModel model)
 {
-    // Counts the bins [base, base + span) of in[0], in[step], in[2 step],
-    // ... (step 1: every tuple); span 32-bit counters in shared memory,
+    // Counts the bins [base, base + span) of one tuple in every `step`
+    // (rj_sample_row; step 1: every tuple); span 32-bit counters in shared memory,
     // stored to this CTA's row of part (rj_hist_sum_kernel adds the rows).
     // With mm: also the key and payload ranges of the tuples read.  MODEL:
     // the bins are the learned model's (rj_model_bin) instead of hash bits.
@@ -61,11 +79,11 @@ __global__ void __launch_bounds__(1024) rj_hist_kernel(const longlong2* __restri
     for (; i + (U - 1) * stride < m; i += U * stride) {
         longlong2 t[U];
 #pragma unroll
-        for (int u = 0; u < U; ++u) t[u] = __ldcs(&in[(i + u * stride) * step]);
+        for (int u = 0; u < U; ++u) t[u] = __ldcs(&in[rj_sample_row(i + u * stride, step, spread, n)]);
 #pragma unroll
         for (int u = 0; u < U; ++u) count(t[u]);
     }
-    for (; i < m; i += stride) count(__ldcs(&in[i * step]));
+    for (; i < m; i += stride) count(__ldcs(&in[rj_sample_row(i, step, spread, n)]));
     if (mm) {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
@@ -327,11 +345,11 @@ __device__ __forceinline__ void rj_load_split(const RJPass& a, long long* dst, i
     for (int i = lane; i < a.nsplit; i += 32) dst[i] = src[i];
 }
 
-// Histogram of range bins of in[0], in[step], ...: fine bin = coarse bin
+// Histogram of range bins of one tuple in every `step`: fine bin = coarse bin
 // (among C - 1 coarse splitters held in shared memory) * 2^sub + bin among
 // that coarse range's 2^sub - 1 fine splitters (read from global memory).
 __global__ void __launch_bounds__(1024) rj_hist_range_kernel(const longlong2* __restrict__ in, int64_t n, int64_t step,
-                                                             int CB, int sub, const long long* __restrict__ csplit,
+                                                             int spread, int CB, int sub, const long long* __restrict__ csplit,
                                                              const long long* __restrict__ fsplit,
                                                              unsigned* __restrict__ part, long long* __restrict__ mm)
 {
@@ -346,7 +364,7 @@ __global__ void __launch_bounds__(1024) rj_hist_range_kernel(const longlong2* __
     long long kmin = LLONG_MAX, kmax = LLONG_MIN, pmin = LLONG_MAX, pmax = LLONG_MIN;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < m; i += stride) {
-        const longlong2 t = __ldcs(&in[i * step]);
+        const longlong2 t = __ldcs(&in[rj_sample_row(i, step, spread, n)]);
         const long long k = t.x;
         kmin = min(kmin, t.x);
         kmax = max(kmax, t.x);
@@ -706,7 +724,7 @@ int launch_pass(pyg_ctx* ctx, const RJPass& p, long long ntiles, bool in8, bool 
 
 // Host-side layout of one relation's partitions.  Exact layouts come from a
 // full histogram (dense, contiguous partitions); sampled layouts size each
-// partition's region from a strided sample with six standard deviations of
+// partition's region from a sample of the rows with six standard deviations of
 
 }  // namespace
 
@@ -919,7 +937,7 @@ int run_passes(pyg_ctx* ctx, const longlong2* in, int64_t n, const RJLayout& L, 
     return launch_pass(ctx, p, ntiles2, L.packed, L.packed);
 }
 
-int hist_launch(pyg_ctx* ctx, const longlong2* in, int64_t n, int64_t step, int FB, unsigned long long* hist,
+int hist_launch(pyg_ctx* ctx, const longlong2* in, int64_t n, int64_t step, int spread, int FB, unsigned long long* hist,
                 long long* mm, const RJModel* model)
 {
     // At most 2^15 counters (128 KB) per launch: 2^16 bins take two.
@@ -943,7 +961,7 @@ int hist_launch(pyg_ctx* ctx, const longlong2* in, int64_t n, int64_t step, int 
     }
     for (int base = 0; base < F; base += span) {
         // The key and payload ranges are taken in the first launch only.
-        kern<<<grid, 1024, hsm, ctx->stream>>>(in, n, step, FB, base, span, part, base ? nullptr : mm,
+        kern<<<grid, 1024, hsm, ctx->stream>>>(in, n, step, spread, FB, base, span, part, base ? nullptr : mm,
                                                 model ? *model : none);
         PYG_LAUNCHED(ctx);
         rj_hist_sum_kernel<<<(span + 255) / 256, 256, 0, ctx->stream>>>(part, grid, span, hist + base);
@@ -953,7 +971,7 @@ int hist_launch(pyg_ctx* ctx, const longlong2* in, int64_t n, int64_t step, int 
     return PYG_OK;
 }
 
-int hist_launch_range(pyg_ctx* ctx, const longlong2* in, int64_t n, int64_t step, int CB, int sub,
+int hist_launch_range(pyg_ctx* ctx, const longlong2* in, int64_t n, int64_t step, int spread, int CB, int sub,
                       const long long* csplit, const long long* fsplit, unsigned long long* hist, long long* mm)
 {
     const int F = 1 << (CB + sub);
@@ -972,7 +990,7 @@ int hist_launch_range(pyg_ctx* ctx, const longlong2* in, int64_t n, int64_t step
         rj_mm_init_kernel<<<1, 32, 0, ctx->stream>>>(mm);
         PYG_LAUNCHED(ctx);
     }
-    rj_hist_range_kernel<<<grid, 1024, hsm, ctx->stream>>>(in, n, step, CB, sub, csplit, fsplit, part, mm);
+    rj_hist_range_kernel<<<grid, 1024, hsm, ctx->stream>>>(in, n, step, spread, CB, sub, csplit, fsplit, part, mm);
     PYG_LAUNCHED(ctx);
     rj_hist_sum_kernel<<<(F + 255) / 256, 256, 0, ctx->stream>>>(part, grid, F, hist);
     PYG_LAUNCHED(ctx);
@@ -1013,10 +1031,10 @@ int rp_partition_sides(pyg_ctx* ctx, RPSide* sd, int ns, int FB, bool two, unsig
     auto hist_of = [&](int s, int64_t st) {
         if (sd[s].csplit) {
             const int cb = coarse_bits(false);
-            return hist_launch_range(ctx, sd[s].in, sd[s].n, st, cb, FB - cb, sd[s].csplit, sd[s].fsplit, hist_at(s),
+            return hist_launch_range(ctx, sd[s].in, sd[s].n, st, two ? 2 : 1, cb, FB - cb, sd[s].csplit, sd[s].fsplit, hist_at(s),
                                      sd[s].allow_pack ? (long long*)(hist_at(s) + F) : nullptr);
         }
-        return hist_launch(ctx, sd[s].in, sd[s].n, st, FB, hist_at(s),
+        return hist_launch(ctx, sd[s].in, sd[s].n, st, two ? 2 : 1, FB, hist_at(s),
                            sd[s].allow_pack ? (long long*)(hist_at(s) + F) : nullptr, sd[s].model);
     };
     // Layout of relation s from host counts h (F counts, then the key and

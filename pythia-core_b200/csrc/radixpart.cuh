@@ -3,7 +3,7 @@
 // operators (join, group-by).
 //
 //   histogram   rj_hist_kernel counts the top `bits` bits of every tuple (or
-//               of a strided sample) in shared memory.
+//               of a sample of the rows) in shared memory.
 //   layout      exact (dense partitions from a full histogram) or sampled
 //               (regions sized from the sample with six standard deviations
 //               of slack; a region that overflows is reported and the caller
@@ -62,7 +62,7 @@ constexpr int RJ_SPLIT_MAX = 256;        // range mode: splitters per pass segme
 // 2^15 32-bit counters in shared memory.
 constexpr int RJ_MAX_FINE_BITS = 16;   // hash mode (histograms run in halves above 2^15 bins)
 constexpr int RJ_MAX_RANGE_BITS = 15;  // range mode (one 2^15-counter histogram)
-// Sampled layouts count every (n >> rj_sample_log2)-th tuple: about 2^9
+// Sampled layouts count one tuple in every n >> rj_sample_log2: about 2^9
 // samples per partition, at most 2^22 (0.1 ms per relation; a sample costs a
 // 32-byte sector, 78 us for 2^22 of 2^27 tuples against 12 us for 2^17).
 // Fewer samples give regions more slack, which costs device memory, not
@@ -163,7 +163,7 @@ struct RJLayout {
 // model: the passes' bins are a learned model's or key ranges.
 void layout_exact(const std::vector<unsigned long long>& h, int64_t n, int C, int sub, RJLayout& L,
                   bool pack = false, bool model = false);
-// Sampled layout from the counts sc of every step-th tuple: each region is
+// Sampled layout from the counts sc of one tuple in every `step`: each region is
 // sized with six standard deviations of slack.
 void layout_sampled(const std::vector<unsigned long long>& sc, long long step, int64_t n, int C, int sub, RJLayout& L,
                     bool pack = false, bool model = false);
@@ -212,11 +212,12 @@ struct RJSideDev {
 
 // Copies a layout to the device and zeroes its cursors.
 int upload_layout(pyg_ctx* ctx, const RJLayout& L, const RJSideDev& d, int F, int C, int64_t n);
-// Histogram of the top FB hash bits of in[0], in[step], ... into hist
+// Histogram of the top FB hash bits of one tuple in every `step` (at a
+// multiple of `spread` inside it, rj_sample_row) into hist
 // (2^FB device words, zeroed here).  mm (optional, 4 words): receives the
 // minimum and maximum key and payload of the tuples read, as signed
 // {kmin, kmax, pmin, pmax}.
-int hist_launch(pyg_ctx* ctx, const longlong2* in, int64_t n, int64_t step, int FB, unsigned long long* hist,
+int hist_launch(pyg_ctx* ctx, const longlong2* in, int64_t n, int64_t step, int spread, int FB, unsigned long long* hist,
                 long long* mm = nullptr, const RJModel* model = nullptr);
 // Partition pass(es) of one relation into P1 (and P2 when two): *err is set
 // if a tile's bulk copy never landed, *ovf if a sampled region overflowed,
@@ -243,8 +244,8 @@ inline size_t pass_bytes(const RJLayout& L, unsigned long long words)
 {
     return ((size_t)words + RJ_DUMP) * elem_bytes(L);
 }
-// Histogram of range bins (see run_passes) of in[0], in[step], ...
-int hist_launch_range(pyg_ctx* ctx, const longlong2* in, int64_t n, int64_t step, int CB, int sub,
+// Histogram of range bins (see run_passes) of one tuple in every `step`.
+int hist_launch_range(pyg_ctx* ctx, const longlong2* in, int64_t n, int64_t step, int spread, int CB, int sub,
                       const long long* csplit, const long long* fsplit, unsigned long long* hist,
                       long long* mm = nullptr);
 // One relation for rp_partition_sides.  In: in, n, allow_sample, the
