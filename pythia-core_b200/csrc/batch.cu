@@ -750,7 +750,8 @@ int pyg_autotune(pyg_ctx* ctx, const pyg_fragment* frags, int32_t n, const char*
     pyg_tuning best_t = default_tuning();
     float best = 1e30f;
     {
-        const int32_t larges[] = {1 << 14, 1 << 16, 1 << 18, 1 << 20};
+        // 0: the default, kLargeBuild within kQueueSlots.
+        const int32_t larges[] = {0, 1 << 14, 1 << 16, 1 << 18, 1 << 20};
         const pyg_tuning base = best_t;
         for (int32_t lb : larges) {
             pyg_tuning t = base;

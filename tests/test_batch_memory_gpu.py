@@ -37,3 +37,18 @@ def test_queued_tables_are_bounded(ctx, torch_cuda):
         assert got == [pyg.PYG_OK] * queued + [pyg.PYG_ERR_ARG] * (len(pairs) - queued)
     finally:
         ctx.batch_free(b)
+
+
+def test_tuner_tries_the_default_threshold(ctx, torch_cuda):
+    """Builds just above 2^20 with few probes: every smaller threshold sends
+    each fragment to a join of its own, whose clear of a table for one
+    fragment at a time is most of the run."""
+    torch = torch_cuda
+    pairs = []
+    for i in range(24):
+        nb, np_ = (1 << 20) + 1 + i, 1024
+        k = torch.randperm(nb, device="cuda")
+        R = torch.stack([k, k], 1).contiguous()
+        pairs.append((R, nb, R[:np_].clone(), np_))
+    t = ctx.autotune(ctx.fragments(pairs), None)
+    assert t.large_build == 0
