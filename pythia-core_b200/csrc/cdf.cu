@@ -127,22 +127,28 @@ __global__ void assign_kernel(const int64_t* __restrict__ keys, int64_t n, doubl
                               LeafStat* __restrict__ st)
 {
     const double a0 = params[0], b0 = params[1];
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        double x = norm_key(keys[i], lo, scale);
-        double r = a0 * x + b0;
-        double fl = floor(L * r);
-        int l = fl < 0 ? 0 : (fl > L - 1 ? L - 1 : (int)fl);
-        double uu = L * r - l;
-        uu = uu < 0 ? 0 : (uu > 1 ? 1 : uu);
-        leaf[i] = l;
-        u[i] = uu;
+    const unsigned lane = threadIdx.x & 31;
+    // Whole warps stay in the loop: the neighbours' leaves are shuffled.
+    for (int64_t wb = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31u); wb < n;
+         wb += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t i = wb + lane;
+        int l = -1;
+        if (i < n) {
+            double x = norm_key(keys[i], lo, scale);
+            double r = a0 * x + b0;
+            double fl = floor(L * r);
+            l = fl < 0 ? 0 : (fl > L - 1 ? L - 1 : (int)fl);
+            double uu = L * r - l;
+            uu = uu < 0 ? 0 : (uu > 1 ? 1 : uu);
+            leaf[i] = l;
+            u[i] = uu;
+        }
         // Only the ends of a warp's runs of one leaf can be its smallest or
         // largest index (the lanes hold consecutive samples): the other
         // lanes' atomics on 1024 leaves took 200 of 240 us for 2^21 samples.
-        const unsigned lane = threadIdx.x & 31, act = __activemask();
-        const int left = __shfl_up_sync(act, l, 1), right = __shfl_down_sync(act, l, 1);
-        if (lane == 0 || left != l) atomicMin(&st[l].lo, (unsigned long long)i);
-        if (lane == 31 || !((act >> (lane + 1)) & 1) || right != l) atomicMax(&st[l].hi, (unsigned long long)(i + 1));
+        const int left = __shfl_up_sync(0xffffffffu, l, 1), right = __shfl_down_sync(0xffffffffu, l, 1);
+        if (l >= 0 && (lane == 0 || left != l)) atomicMin(&st[l].lo, (unsigned long long)i);
+        if (l >= 0 && (lane == 31 || right != l)) atomicMax(&st[l].hi, (unsigned long long)(i + 1));
     }
 }
 
