@@ -69,7 +69,12 @@ __global__ void __launch_bounds__(BS_THREADS) bs_page_kernel(const uint64_t* __r
     if (tid == 0 && 2 * units < cnt) page[cnt - 1] = in[base + cnt - 1];  // odd last record
     __syncthreads();
     if (!ok) {
-        if (tid == 0) atomicOr(err, 1u);
+        if (tid == 0) {
+            atomicOr(err, 1u);
+            // The copy gets as long again to land before this CTA's shared
+            // memory is given up.
+            mbar_wait(&bar, 0, kBsWaitNs);
+        }
         return;
     }
     // Order-preserving flip of the records; padding is the largest item.

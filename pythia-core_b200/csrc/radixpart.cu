@@ -487,7 +487,17 @@ __global__ void __launch_bounds__(RJShape<IN8, OUT8, MODE>::THREADS, RJShape<IN8
         long long k = 0;
         for (long long tile = blockIdx.x;; tile += gridDim.x, ++k) {
             __syncthreads();  // 1
-            if (!sm.ok || tile >= ntiles) break;
+            if (!sm.ok || tile >= ntiles) {
+                // A wait ran out: copies still in flight get as long again to
+                // land before this CTA's shared memory is given up.
+                if (ct == 0 && !sm.ok) {
+                    atomicOr(a.err, 1u);
+                    for (int s = 0; s < ST; ++s)
+                        if (tile + (long long)s * gridDim.x < ntiles)
+                            mbar_wait(&sm.bar[(k + s) % ST], (unsigned)(((k + s) / ST) & 1), kBulkWaitNs);
+                }
+                break;
+            }
             const int slot = (int)(k % ST);
             unsigned* hist = sm.hist[k & 1];
             if (first) {
@@ -574,7 +584,6 @@ __global__ void __launch_bounds__(RJShape<IN8, OUT8, MODE>::THREADS, RJShape<IN8
                 }
             }
         }
-        if (ct == 0 && !sm.ok) atomicOr(a.err, 1u);
         return;
     }
     // ---- workers
