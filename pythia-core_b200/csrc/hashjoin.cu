@@ -234,21 +234,14 @@ __device__ __forceinline__ void block_flush(uint64_t* acc, int nacc, unsigned lo
 // match count, the build-payload sum and the probe-value sum.  FILLERS:
 // tuples whose key is the empty marker are padding (skipped) rather than
 // real keys (matched against the side list).
-#ifndef PYG_PROBE_UNROLL
-#define PYG_PROBE_UNROLL 4
-#endif
-#ifndef PYG_PROBE_MIN_BLOCKS
-#define PYG_PROBE_MIN_BLOCKS 4
-#endif
-
 template <int UNROLL, bool FILLERS>
-__global__ void __launch_bounds__(256, PYG_PROBE_MIN_BLOCKS) probe_agg16_kernel(const longlong2* __restrict__ S, int64_t n,
-                                                          const ulonglong2* __restrict__ slots, uint64_t cap,
-                                                          const unsigned long long* __restrict__ counts,
-                                                          const uint64_t* __restrict__ side, int64_t nside,
-                                                          unsigned long long* __restrict__ out,
-                                                          const unsigned long long* __restrict__ gate,
-                                                          int64_t side_cap)
+__global__ void __launch_bounds__(256, 4) probe_agg16_kernel(const longlong2* __restrict__ S, int64_t n,
+                                                             const ulonglong2* __restrict__ slots, uint64_t cap,
+                                                             const unsigned long long* __restrict__ counts,
+                                                             const uint64_t* __restrict__ side, int64_t nside,
+                                                             unsigned long long* __restrict__ out,
+                                                             const unsigned long long* __restrict__ gate,
+                                                             int64_t side_cap)
 {
     // gate (optional): the build's flags, read here instead of on the host.
     // A build with repeated keys (no count array), a full table or more
@@ -617,7 +610,7 @@ static int launch_probe16(pyg_ctx* ctx, const pyg_hashtable* ht, const longlong2
 {
     if (n <= 0) return PYG_OK;
     int threads = 256;
-    constexpr int U = PYG_PROBE_UNROLL;
+    constexpr int U = 4;
     int grid = grid_for(ctx, n, threads, U, 8);
     if (fillers)
         probe_agg16_kernel<U, true><<<grid, threads, 0, ctx->stream>>>(S, n, (const ulonglong2*)ht->slots, ht->cap,
@@ -708,10 +701,7 @@ struct PhaseTimer {
 // probe keys equal to it are matched against that list.
 
 constexpr int DJ_THREADS = 256;
-#ifndef PYG_DJ_UNROLL
-#define PYG_DJ_UNROLL 4
-#endif
-constexpr int DJ_U = PYG_DJ_UNROLL;
+constexpr int DJ_U = 4;
 
 __device__ __forceinline__ uint64_t dj_slot(uint64_t k, int shift) { return rj_hash(k) >> shift; }
 

@@ -39,30 +39,15 @@
 
 namespace pyg {
 
-#ifndef PYG_RJ_JOIN_THREADS
-#define PYG_RJ_JOIN_THREADS 1024
-#endif
-#ifndef PYG_RJ_JOIN_BLOCKS
-#define PYG_RJ_JOIN_BLOCKS 1
-#endif
-#ifndef PYG_RJ_TABLE_KB
-#define PYG_RJ_TABLE_KB 192
-#endif
-#ifndef PYG_RJ_RCAP_PCT
-#define PYG_RJ_RCAP_PCT 50
-#endif
-constexpr int RJ_JOIN_THREADS = PYG_RJ_JOIN_THREADS;
-constexpr int RJ_JOIN_BLOCKS = PYG_RJ_JOIN_BLOCKS;  // join CTAs per SM
-#ifndef PYG_RJ_PROBE_UNROLL
-#define PYG_RJ_PROBE_UNROLL 4
-#endif
-constexpr int RJ_PROBE_UNROLL = PYG_RJ_PROBE_UNROLL;  // probe tuples in flight per thread
-constexpr int RJ_TABLE_BYTES = PYG_RJ_TABLE_KB * 1024;
+constexpr int RJ_JOIN_THREADS = 1024;
+constexpr int RJ_JOIN_BLOCKS = 1;   // join CTAs per SM
+constexpr int RJ_PROBE_UNROLL = 4;  // probe tuples in flight per thread
+constexpr int RJ_TABLE_BYTES = 192 * 1024;
 constexpr int RJ_SLOTS_UNIQUE = RJ_TABLE_BYTES / 16;   // {key, payload}
 constexpr int RJ_SLOTS_COUNTED = RJ_TABLE_BYTES / 32;  // {key, payload sum, count, -}
-// Build tuples per work item: at most this share of the table's slots.
-constexpr unsigned RJ_RCAP_UNIQUE = RJ_SLOTS_UNIQUE * PYG_RJ_RCAP_PCT / 100;
-constexpr unsigned RJ_RCAP_COUNTED = RJ_SLOTS_COUNTED * PYG_RJ_RCAP_PCT / 100;
+// Build tuples per work item: at most half the table's slots.
+constexpr unsigned RJ_RCAP_UNIQUE = RJ_SLOTS_UNIQUE / 2;
+constexpr unsigned RJ_RCAP_COUNTED = RJ_SLOTS_COUNTED / 2;
 constexpr int64_t RJ_SCHUNK = 1 << 16;                 // probe tuples per work item (at most)
 
 // ---------------------------------------------------------------------------
@@ -348,26 +333,14 @@ __global__ void __launch_bounds__(RJ_JOIN_THREADS, RJ_JOIN_BLOCKS) rj_join_kerne
 // Buckets of two words measured 3.21 ms (random hash) and 2.59 ms (even
 // slots).
 
-#ifndef PYG_RJ32_TABLE_KB
-#define PYG_RJ32_TABLE_KB 96
-#endif
-#ifndef PYG_RJ32_BLOCKS
-#define PYG_RJ32_BLOCKS 2
-#endif
 constexpr int RJ32_THREADS = 1024;
-constexpr int RJ32_BLOCKS = PYG_RJ32_BLOCKS;  // CTAs per SM
-constexpr int RJ32_TABLE_BYTES = PYG_RJ32_TABLE_KB * 1024;
+constexpr int RJ32_BLOCKS = 2;  // CTAs per SM
+constexpr int RJ32_TABLE_BYTES = 96 * 1024;
 constexpr unsigned RJ32_SLOTS = RJ32_TABLE_BYTES / 8;
 constexpr unsigned RJ32_RCAP = RJ32_SLOTS / 2;
-#ifndef PYG_RJ32_U
-#define PYG_RJ32_U 8
-#endif
-#ifndef PYG_RJ32_PREFETCH
-#define PYG_RJ32_PREFETCH 8192
-#endif
-constexpr int RJ32_U = PYG_RJ32_U;  // probe words in flight per thread
+constexpr int RJ32_U = 8;  // probe words in flight per thread
 // Words of the next item's probe chunk pulled into L2 ahead of use.
-constexpr unsigned RJ32_PREFETCH = PYG_RJ32_PREFETCH;
+constexpr unsigned RJ32_PREFETCH = 8192;
 constexpr unsigned long long kEmptyWord = ~0ULL;
 
 __global__ void __launch_bounds__(RJ32_THREADS, RJ32_BLOCKS) rj_join32_kernel(RJJoinArgs a)

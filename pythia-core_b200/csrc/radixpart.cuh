@@ -47,12 +47,13 @@ constexpr int RJ_SM_LEAVES = 1024;
 constexpr int RJ_SM_HEAVY = 512;
 constexpr int RJ_TILE_MIN = 1024;
 // Tile of a pass over n elements: the largest, halved until a pass has about
-// two tiles for each of 148 SMs (small relations would otherwise leave SMs
-// without a tile).
+// two tiles for each of the 148 SMs (small relations would otherwise leave
+// SMs without a tile).
+constexpr int64_t RJ_TILES_MIN = 2 * 148;
 inline int rj_tile(int largest, int64_t n)
 {
     int t = largest;
-    while (t > RJ_TILE_MIN && n < (int64_t)t * 296) t = (t >> 1) & ~1;  // even: tiles of packed words start 16-byte aligned
+    while (t > RJ_TILE_MIN && n < t * RJ_TILES_MIN) t = (t >> 1) & ~1;  // even: tiles of packed words start 16-byte aligned
     return t;
 }
 constexpr int RJ_MAX_LOCAL_BITS = 9;     // bins of one partition pass

@@ -156,20 +156,11 @@ __device__ __forceinline__ uint64_t os_key(const Item& t)
 }
 
 // Threads and elements per thread of a pass's CTA.
-#ifndef PYG_OS_T16
-#define PYG_OS_T16 512
-#endif
-#ifndef PYG_OS_I16
-#define PYG_OS_I16 8
-#endif
-#ifndef PYG_OS_MINB16
-#define PYG_OS_MINB16 2
-#endif
 template <typename Item>
 struct OsShape {
-    static constexpr int THREADS = sizeof(Item) == 16 ? PYG_OS_T16 : 512;
-    static constexpr int PER = sizeof(Item) == 16 ? PYG_OS_I16 : 12;
-    static constexpr int MINB = sizeof(Item) == 16 ? PYG_OS_MINB16 : 2;
+    static constexpr int THREADS = 512;
+    static constexpr int PER = sizeof(Item) == 16 ? 8 : 12;
+    static constexpr int MINB = 2;
     static constexpr int TILE = THREADS * PER;
     static constexpr int WARPS = THREADS / 32;
     static constexpr size_t COUNTERS = (size_t)WARPS * OS_BINS * 4;
