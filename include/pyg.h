@@ -212,8 +212,9 @@ typedef struct pyg_join_stats {
     double probe_pass_ms[2];
     int32_t build_packed;       /* 8-byte packed intermediates (RADIX)  */
     int32_t probe_packed;
-    /* RADIX: the join kernel alone; probe_ms also holds the host round trip
-     * that reads the partition counts and uploads the work items. */
+    /* RADIX: the join kernel alone; probe_ms also holds the forming of its
+     * work items (on the device, or on the host for partitions that are cut
+     * on both sides beyond the device's list). */
     double join_kernel_ms;
 } pyg_join_stats;
 

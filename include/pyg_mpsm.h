@@ -6,11 +6,12 @@
  * that feeds them (PartitionOp with exactrange, operators/partition.cpp,
  * and the buildprepartitioned option, join.cpp:1002-1009, :1266-1283).
  *
- * Both inputs are range-partitioned by the same splitters (equal-width as
- * the reference's ExactRangeValueHasher, quantiles of a key sample, or the
- * learned CDF model), each partition is sorted (4 KB pages bitonic-sorted
- * in shared memory, then merge-path merge rounds), and matching partitions
- * are merge-joined.  Single join key column per side (int32 or int64).
+ * Aggregate sink: both inputs are range-partitioned by the same splitters
+ * (equal-width as the reference's ExactRangeValueHasher, quantiles of a key
+ * sample, or the learned CDF model), each partition is sorted in shared
+ * memory, and matching partitions are merge-joined.  Materialising sink: both
+ * inputs are sorted as a whole and merged, without range partitions.  Single
+ * join key column per side (int32 or int64).
  */
 #ifndef PYG_MPSM_H
 #define PYG_MPSM_H
@@ -51,8 +52,9 @@ int pyg_mpsm_join_agg(pyg_ctx* ctx, const pyg_rel* build, int32_t build_key, con
 
 /* Materialising variant into a device buffer of out_capacity tuples
  * (projected columns packed).  Output order: ascending key, then probe
- * input position, then build input position.  PYG_ERR_CAPACITY (with
- * *out_count set) when the result does not fit. */
+ * input position, then build input position.  The options are checked as for
+ * the aggregate sink but choose nothing here (no splitters, no model).
+ * PYG_ERR_CAPACITY (with *out_count set) when the result does not fit. */
 int pyg_mpsm_join_materialize(pyg_ctx* ctx, const pyg_rel* build, int32_t build_key,
                               const pyg_rel* probe, int32_t probe_key, const pyg_proj* proj,
                               int32_t nproj, const pyg_mpsm_opts* opts, void* out,

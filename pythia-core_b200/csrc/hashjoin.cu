@@ -806,8 +806,9 @@ __device__ __forceinline__ void dj_match(const longlong2 t, ulonglong2 e, uint64
 // so this launch then does nothing.  host (optional, pinned): the last CTA
 // to finish copies the 11 counter words there (words = flags, words[11] its
 // zeroed ticket; out lies in words, so neither is __restrict__), in place of
-// a device-to-host copy after the kernel: 2^20 x 2^24 141.2 -> 138.8 us,
-// 20 K x 400 K 41.3 -> 35.2, 100 K x 1 M 47.7 -> 45.8.
+// a device-to-host copy after the kernel: 20 K x 400 K 41.3 -> 35.2 us,
+// 100 K x 1 M 47.7 -> 45.8; at 2^20 x 2^24 the difference (141 and 139 us) lies
+// within the spread of the calls.
 // Bound: one table sector per clock and SM through L1 (16.7 M probes: 57 us
 // of the 87).
 __global__ void __launch_bounds__(DJ_THREADS) dj_probe_kernel(const longlong2* __restrict__ S, int64_t n,

@@ -1,9 +1,10 @@
-// Decoupled look-back: tiles of one kernel learn what precedes them from
-// their predecessors' status words.  A tile's word is a single 64-bit store
-// that carries a flag and a value, so relaxed accesses suffice.  Tiles are
-// numbered by a ticket that running CTAs draw: a tile waits only for tiles
-// whose CTAs are already running and never wait for it, so every wait ends;
-// the waits are bounded all the same and report an error.
+// Decoupled look-back (Merrill and Garland, "Single-pass Parallel Prefix Scan
+// with Decoupled Look-back", 2016): tiles of one kernel learn what precedes
+// them from their predecessors' status words.  A tile's word is a single
+// 64-bit store that carries a flag and a value, so relaxed accesses suffice.
+// Tiles are numbered by a ticket that running CTAs draw: a tile waits only for
+// tiles whose CTAs are already running and never wait for it, so every wait
+// ends; the waits are bounded all the same and report an error.
 #pragma once
 #include <stdint.h>
 

@@ -118,7 +118,9 @@ int exclusive_scan_u64(pyg_ctx* ctx, const unsigned long long* in, unsigned long
 }
 
 // ---------------------------------------------------------------------------
-// Stable LSD radix sort in one sweep per 8-bit digit.
+// Stable LSD radix sort in one sweep per 8-bit digit, the published Onesweep
+// scheme (Adinets and Merrill, "Onesweep: A Faster Least Significant Digit
+// Radix Sort for GPUs", 2022).
 //
 //   range   one read takes the smallest and largest key; digits are those of
 //           key - smallest, so only the bits the keys span are sorted (a
@@ -142,7 +144,10 @@ int exclusive_scan_u64(pyg_ctx* ctx, const unsigned long long* in, unsigned long
 // 1234; 512 x 6, 2: 1243; 256 x 16, 3 and 512 x 12, 2 spill registers
 // (1311, 1283).
 //
-// The waits of the look-back are bounded (lookback.cuh).
+// The waits of the look-back are bounded (lookback.cuh).  A wait that gives up
+// sets the context's sort error word, and nothing that was queued behind it
+// touches the unfinished order: passes, gathers and merges look at the word
+// first.
 
 constexpr int OS_BINS = 256;
 constexpr int OS_MAX_PASSES = 8;

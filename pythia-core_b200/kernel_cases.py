@@ -19,6 +19,8 @@ device.  Cases and the kernels they launch:
   sort       2^24 tuples                            os_range, os_hist, os_pass
   mpsm       R 2^22 x S 2^24, sampled or learned splitters   mp16 path (aggregate sink)
   mpsm-mat   R 2^20 x S 2^22, materialised          os_pass, mm_join
+  rows       R 2^20 x S 2^23 joined rows               ht_build16, probe_mat16
+  small      R 4096 x S 2^24 join                      sj
   cdf        2^21-key sample, 1024 leaves           cdf training kernels
   batch      64 fragments, builds 2^12..2^18        batch_kernel
 """
@@ -137,6 +139,18 @@ def case_mpsm(torch, ctx, a, materialize):
             assert cnt == nS and (sb + sp) & 0xFFFFFFFFFFFFFFFF == want
 
 
+def case_rows(torch, ctx, a):
+    nR, nS = (1 << 20) >> a.shift, (1 << 23) >> a.shift
+    R, S = pkfk(torch, ctx, nR, nS, a.theta)
+    Rr, Sr = pyg.Rel(R, nR, [I64, I64]), pyg.Rel(S, nS, [I64, I64])
+    out = torch.empty(nS * 2, dtype=torch.int64, device="cuda")
+    for _ in range(a.reps):
+        ht = ctx.hashjoin_build(Rr, [0], [1], pyg.HT_MATERIALIZE, 0.5)
+        rc, cnt = ctx.hashjoin_probe_materialize(ht, Sr, [0], [(0, 1), (1, 1)], out, nS)
+        ht.free()
+        assert rc == 0 and cnt == nS
+
+
 def case_cdf(torch, ctx, a):
     n = (1 << 21) >> a.shift
     keys = torch.sort(torch.randint(-(1 << 40), 1 << 40, (n,), device="cuda"))[0]
@@ -172,7 +186,7 @@ def case_batch(torch, ctx, a):
 def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("case", choices=["radix", "direct", "groupby16", "groupby-zipf", "composite", "partition", "sort", "mpsm",
-                                     "mpsm-mat", "cdf", "batch"])
+                                     "mpsm-mat", "rows", "small", "cdf", "batch"])
     ap.add_argument("--shift", type=int, default=0, help="shrink the inputs by 2^shift")
     ap.add_argument("--reps", type=int, default=2)
     ap.add_argument("--theta", type=float, default=0.0)
@@ -201,6 +215,10 @@ def main():
             case_sort(torch, ctx, a)
         elif a.case in ("mpsm", "mpsm-mat"):
             case_mpsm(torch, ctx, a, a.case == "mpsm-mat")
+        elif a.case == "rows":
+            case_rows(torch, ctx, a)
+        elif a.case == "small":
+            case_join(torch, ctx, a, pyg.JOIN_DIRECT, 4096, (1 << 24) >> a.shift)
         elif a.case == "cdf":
             case_cdf(torch, ctx, a)
         else:
