@@ -160,7 +160,10 @@ int partition_device(pyg_ctx* ctx, const pyg_rel* in, int32_t key_col, const Buc
                           ? (size_t)(f.fanout - 1) * 8 : 0;
     size_t hist_smem = (((size_t)f.fanout * 4 + 15) & ~(size_t)15) + spl_smem;
     size_t scat_smem = (size_t)f.fanout * 8 + spl_smem;
-    if (scat_smem > 200 * 1024 || hist_smem > 200 * 1024) {
+    // The kernels' limit, set for the largest call: the attribute is the
+    // process's, and a call on another thread may launch in between.
+    constexpr int kMaxSmem = 200 * 1024;
+    if (scat_smem > kMaxSmem || hist_smem > kMaxSmem) {
         set_error("partition: fan-out %u too large for one pass", f.fanout);
         return PYG_ERR_ARG;
     }
@@ -171,7 +174,7 @@ int partition_device(pyg_ctx* ctx, const pyg_rel* in, int32_t key_col, const Buc
     PYG_CUDA(cudaMemsetAsync(err, 0, 8, ctx->stream));
     int32_t off = in->col_offset[key_col], type = in->col_type[key_col];
     const uint8_t* base = (const uint8_t*)in->base;
-    PYG_CUDA(cudaFuncSetAttribute(pt_hist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hist_smem));
+    PYG_CUDA(cudaFuncSetAttribute(pt_hist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem));
     pt_hist_kernel<<<blocks, threads, hist_smem, ctx->stream>>>(base, n, in->tuple_bytes, off, type, f, chunk, hist, err);
     PYG_LAUNCHED(ctx);
     unsigned long long* h = (unsigned long long*)ctx->pinned + 72;
@@ -192,16 +195,16 @@ int partition_device(pyg_ctx* ctx, const pyg_rel* in, int32_t key_col, const Buc
     bool a4 = tb % 4 == 0 && (uintptr_t)base % 4 == 0 && (uintptr_t)out % 4 == 0;
     if (n > 0) {
         if (a16) {
-            PYG_CUDA(cudaFuncSetAttribute(pt_scatter_kernel<uint4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scat_smem));
+            PYG_CUDA(cudaFuncSetAttribute(pt_scatter_kernel<uint4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem));
             pt_scatter_kernel<uint4><<<blocks, threads, scat_smem, ctx->stream>>>(base, n, tb, off, type, f, chunk, hist, (uint8_t*)out);
         } else if (a8) {
-            PYG_CUDA(cudaFuncSetAttribute(pt_scatter_kernel<uint2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scat_smem));
+            PYG_CUDA(cudaFuncSetAttribute(pt_scatter_kernel<uint2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem));
             pt_scatter_kernel<uint2><<<blocks, threads, scat_smem, ctx->stream>>>(base, n, tb, off, type, f, chunk, hist, (uint8_t*)out);
         } else if (a4) {
-            PYG_CUDA(cudaFuncSetAttribute(pt_scatter_kernel<unsigned>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scat_smem));
+            PYG_CUDA(cudaFuncSetAttribute(pt_scatter_kernel<unsigned>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem));
             pt_scatter_kernel<unsigned><<<blocks, threads, scat_smem, ctx->stream>>>(base, n, tb, off, type, f, chunk, hist, (uint8_t*)out);
         } else {
-            PYG_CUDA(cudaFuncSetAttribute(pt_scatter_kernel<unsigned char>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scat_smem));
+            PYG_CUDA(cudaFuncSetAttribute(pt_scatter_kernel<unsigned char>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem));
             pt_scatter_kernel<unsigned char><<<blocks, threads, scat_smem, ctx->stream>>>(base, n, tb, off, type, f, chunk, hist, (uint8_t*)out);
         }
         PYG_LAUNCHED(ctx);

@@ -954,7 +954,9 @@ int hist_launch(pyg_ctx* ctx, const longlong2* in, int64_t n, int64_t step, int 
     const size_t hsm = (size_t)4 * span;
     auto kern = model ? rj_hist_kernel<true> : rj_hist_kernel<false>;
     const RJModel none;
-    PYG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hsm));
+    // The most that any call needs: the attribute is the process's, and a call
+    // on another thread may launch the kernel between these lines.
+    PYG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 << 15));
     int per = 0;
     PYG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, 1024, hsm));
     if (per < 1) per = 1;
@@ -985,7 +987,8 @@ int hist_launch_range(pyg_ctx* ctx, const longlong2* in, int64_t n, int64_t step
 {
     const int F = 1 << (CB + sub);
     const size_t hsm = (size_t)RJ_SPLIT_MAX * 8 + (size_t)4 * F;
-    PYG_CUDA(cudaFuncSetAttribute(rj_hist_range_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hsm));
+    PYG_CUDA(cudaFuncSetAttribute(rj_hist_range_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  RJ_SPLIT_MAX * 8 + (4 << RJ_MAX_RANGE_BITS)));  // as in hist_launch
     int per = 0;
     PYG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, rj_hist_range_kernel, 1024, hsm));
     if (per < 1) per = 1;
