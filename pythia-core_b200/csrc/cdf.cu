@@ -67,6 +67,13 @@ __device__ __forceinline__ double norm_key(int64_t k, double lo, double scale)
     return (double)(float)(((double)k - lo) * scale);
 }
 
+// Leaf of root value r: floor(L r) within [0, L - 1], and 0 for NaN.
+__host__ __device__ __forceinline__ int leaf_of(double r, int L)
+{
+    const double fl = floor(L * r);
+    return fl > 0 ? (fl < L ? (int)fl : L - 1) : 0;
+}
+
 // Root forward + backward over the sorted sample: acc[0] += e^2,
 // acc[1] += e*x, acc[2] += e with e = a0*x + b0 - y.
 __global__ void __launch_bounds__(CDF_THREADS) root_fwd_bwd_kernel(const int64_t* __restrict__ keys, int64_t n,
@@ -136,8 +143,7 @@ __global__ void assign_kernel(const int64_t* __restrict__ keys, int64_t n, doubl
         if (i < n) {
             double x = norm_key(keys[i], lo, scale);
             double r = a0 * x + b0;
-            double fl = floor(L * r);
-            l = fl < 0 ? 0 : (fl > L - 1 ? L - 1 : (int)fl);
+            l = leaf_of(r, L);
             double uu = L * r - l;
             uu = uu < 0 ? 0 : (uu > 1 ? 1 : uu);
             leaf[i] = l;
@@ -339,8 +345,7 @@ __global__ void predict_kernel(const int64_t* __restrict__ keys, int64_t n, doub
         const int64_t k = keys[i];
         double x = norm_key(k, lo, scale);
         double r = a0 * x + b0;
-        double fl = floor(L * r);
-        int l = fl < 0 ? 0 : (fl > L - 1 ? L - 1 : (int)fl);
+        const int l = leaf_of(r, L);
         double uu = L * r - l;
         uu = uu < 0 ? 0 : (uu > 1 ? 1 : uu);
         double f = (double)params[2 + 2 * l] * uu + (double)params[3 + 2 * l];
@@ -635,7 +640,10 @@ int pyg_cdf_train(pyg_ctx* ctx, const int64_t* sample_keys, int64_t n, const pyg
                                      ctx->stream));
         }
         m->key_lo = (double)m->kmin;
-        m->key_scale = m->kmax > m->kmin ? 1.0 / ((double)m->kmax - (double)m->kmin) : 0.0;
+        // A range that vanishes in doubles (a few hundred keys at either end
+        // of int64) has no scale, like one key value.
+        const double range = (double)m->kmax - (double)m->kmin;
+        m->key_scale = range > 0 ? 1.0 / range : 0.0;
 
         // Initial parameters: root y = x, leaves t = u.
         std::vector<float> p(2 + 2 * L);
@@ -734,8 +742,7 @@ static double cdf_continuous(const pyg_cdf* m, int64_t k)
     const double x = (double)(float)(((double)k - m->key_lo) * m->key_scale);
     const double r = (double)m->a0 * x + (double)m->b0;
     const int L = m->L;
-    const double fl = floor(L * r);
-    const int l = fl < 0 ? 0 : (fl > L - 1 ? L - 1 : (int)fl);
+    const int l = leaf_of(r, L);
     double uu = L * r - l;
     uu = uu < 0 ? 0 : (uu > 1 ? 1 : uu);
     double f = (double)m->la[l] * uu + (double)m->lb[l];
