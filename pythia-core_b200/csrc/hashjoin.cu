@@ -925,12 +925,12 @@ bool direct_join16_result(const unsigned long long* w, int64_t nR, unsigned long
 // SM).  4096 x 65536 tuples: 28 us a call, 12 of them the kernel, against 40 us
 // with three launches, a copy and a wait.
 constexpr int SJ_THREADS = 1024;
-constexpr int SJ_MAX_BITS = 13;                       // 8192 slots of 16 bytes
-constexpr int64_t SJ_MAX_BUILD = 6 * SJ_THREADS;      // load factor 0.75
-constexpr int SJ_PINNED = 2048;                       // word of the pinned area where the CTAs' sums begin
+constexpr unsigned SJ_MIN_SLOTS = 256, SJ_MAX_SLOTS = 14336;  // 16 bytes each: at most 224 KB
+constexpr int64_t SJ_MAX_BUILD = 6 * SJ_THREADS;              // load factor 0.43
+constexpr int SJ_PINNED = 2048;                               // word of the pinned area where the CTAs' sums begin
 
 __global__ void __launch_bounds__(SJ_THREADS, 1) sj_kernel(const longlong2* __restrict__ R, int nR,
-                                                           const longlong2* __restrict__ S, int64_t nS, int bits,
+                                                           const longlong2* __restrict__ S, int64_t nS, unsigned cap,
                                                            unsigned long long* __restrict__ host)
 {
     // host: this CTA's {matches, build sum, probe sum, a repeated build key}.
@@ -940,8 +940,7 @@ __global__ void __launch_bounds__(SJ_THREADS, 1) sj_kernel(const longlong2* __re
     __shared__ unsigned dupf;
     constexpr int U = 4, RB = (int)(SJ_MAX_BUILD / SJ_THREADS);
     const int tid = threadIdx.x;
-    const unsigned cap = 1u << bits, mask = cap - 1;
-    const int shift = 64 - bits;
+    auto slot = [&](unsigned long long k) { return __umulhi((unsigned)(rj_hash(k) >> 32), cap); };
     // The build tuples and the first probe tuples are on their way while the
     // table is cleared.
     longlong2 r[RB], t[U];
@@ -969,7 +968,7 @@ __global__ void __launch_bounds__(SJ_THREADS, 1) sj_kernel(const longlong2* __re
             atomicAdd(&side_sum, (unsigned long long)r[j].y);
             continue;
         }
-        unsigned pos = (unsigned)dj_slot(k, shift);
+        unsigned pos = slot(k);
         for (unsigned steps = 0; steps < cap; ++steps) {
             const unsigned long long prev = atomicCAS(&T[pos].x, kEmptyKey, k);
             if (prev == kEmptyKey) {
@@ -980,7 +979,7 @@ __global__ void __launch_bounds__(SJ_THREADS, 1) sj_kernel(const longlong2* __re
                 dup = true;
                 break;
             }
-            pos = (pos + 1) & mask;
+            pos = pos + 1 == cap ? 0 : pos + 1;
         }
     }
     if (dup) dupf = 1;
@@ -995,7 +994,7 @@ __global__ void __launch_bounds__(SJ_THREADS, 1) sj_kernel(const longlong2* __re
             psum += scnt * (uint64_t)x.y;
             return;
         }
-        unsigned pos = (unsigned)dj_slot(k, shift);
+        unsigned pos = slot(k);
         for (unsigned steps = 0; steps < cap; ++steps) {
             const ulonglong2 e = T[pos];
             if (e.x == k) {
@@ -1005,7 +1004,7 @@ __global__ void __launch_bounds__(SJ_THREADS, 1) sj_kernel(const longlong2* __re
                 return;
             }
             if (e.x == kEmptyKey) return;
-            pos = (pos + 1) & mask;
+            pos = pos + 1 == cap ? 0 : pos + 1;
         }
     };
     while (i < nS) {
@@ -1050,13 +1049,17 @@ static int direct_join16(pyg_ctx* ctx, const longlong2* R, int64_t nR, const lon
     // Phase times need the three launches.  Load factors that no table
     // accepts keep to them too, where one that leaves no room is refused.
     if (nR <= SJ_MAX_BUILD && !tm->on && lf <= 0.95f) {
-        int bits = 8;
-        while (bits < SJ_MAX_BITS && ((int64_t)1 << bits) < 2 * nR) ++bits;
-        PYG_CUDA(cudaFuncSetAttribute(sj_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 16 << SJ_MAX_BITS));
+        // Four slots per tuple where they fit: the longest of a warp's 32
+        // chains decides its lookups.  Random 31-bit keys, half of the 20 M
+        // probes matched: 165 us for 6144 build tuples and 110 for 256, where
+        // two slots per tuple (at most 8192) took 620 and 183 and the three
+        // launches 198 and 124.
+        const unsigned slots = (unsigned)std::min<int64_t>(SJ_MAX_SLOTS, std::max<int64_t>(SJ_MIN_SLOTS, 4 * nR));
+        PYG_CUDA(cudaFuncSetAttribute(sj_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 16 * SJ_MAX_SLOTS));
         const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(ctx->sm_count, (nS + SJ_THREADS - 1) / SJ_THREADS));
         static_assert(SJ_PINNED * 8 + 1024 * 32 <= kPinnedScalarBytes, "the CTAs' sums fit the scalar area");
         unsigned long long* part = h + SJ_PINNED;
-        sj_kernel<<<std::min(grid, 1024), SJ_THREADS, 16 << bits, ctx->stream>>>(R, (int)nR, S, nS, bits, part);
+        sj_kernel<<<std::min(grid, 1024), SJ_THREADS, 16 * slots, ctx->stream>>>(R, (int)nR, S, nS, slots, part);
         PYG_LAUNCHED(ctx);
         PYG_CUDA(cudaStreamSynchronize(ctx->stream));
         unsigned long long dups = 0;
