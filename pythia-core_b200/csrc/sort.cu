@@ -122,9 +122,10 @@ int exclusive_scan_u64(pyg_ctx* ctx, const unsigned long long* in, unsigned long
 // scheme (Adinets and Merrill, "Onesweep: A Faster Least Significant Digit
 // Radix Sort for GPUs", 2022).
 //
-//   range   one read takes the smallest and largest key; digits are those of
-//           key - smallest, so only the bits the keys span are sorted (a
-//           signed 40-bit range takes 5 passes, not 8).
+//   range   one read takes the smallest and largest key and the low bits that
+//           all keys share; digits are those of key - smallest above these, so
+//           only the bits the keys span are sorted (a signed 40-bit range
+//           takes 5 passes, not 8; 256 multiples of 2^56 take one).
 //   hist    one read counts every pass's digits (shared-memory counters).
 //   pass    each CTA takes a tile by ticket, ranks it by digit, learns how
 //           many elements of each digit precede the tile from its
@@ -175,18 +176,20 @@ struct OsShape {
 
 // Smallest and largest key, each as an atomicMin (words start at all ones):
 // words[0] the smallest order-preserving image, words[1] the complement of
-// the largest.
+// the largest; words[2] the bits in which all keys are equal.
 template <typename Item, int FIELD>
 __global__ void __launch_bounds__(512) os_range_kernel(const Item* __restrict__ in, int64_t n, uint64_t flip,
                                                        unsigned long long* __restrict__ words)
 {
-    unsigned long long lo = ~0ULL, hi = ~0ULL;
+    unsigned long long lo = ~0ULL, hi = ~0ULL, diff = 0;
+    const unsigned long long first = os_key<Item, FIELD>(in[0]) ^ flip;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     auto take = [&](const Item& t) {
         const unsigned long long k = os_key<Item, FIELD>(t) ^ flip;
         lo = min(lo, k);
         hi = min(hi, ~k);
+        diff |= k ^ first;
     };
     constexpr int U = 4;
     for (; i + (U - 1) * stride < n; i += U * stride) {
@@ -201,17 +204,20 @@ __global__ void __launch_bounds__(512) os_range_kernel(const Item* __restrict__ 
     for (int o = 16; o > 0; o >>= 1) {
         lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
         hi = min(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+        diff |= __shfl_xor_sync(0xffffffffu, diff, o);
     }
-    __shared__ unsigned long long red[2][16];
+    __shared__ unsigned long long red[3][16];
     if ((threadIdx.x & 31) == 0) {
         red[0][threadIdx.x >> 5] = lo;
         red[1][threadIdx.x >> 5] = hi;
+        red[2][threadIdx.x >> 5] = ~diff;
     }
     __syncthreads();
-    if (threadIdx.x < 2) {
+    if (threadIdx.x < 3) {
         unsigned long long m = ~0ULL;
-        for (int w = 0; w < 16; ++w) m = min(m, red[threadIdx.x][w]);
-        atomicMin(&words[threadIdx.x], m);
+        for (int w = 0; w < 16; ++w) m = threadIdx.x < 2 ? min(m, red[threadIdx.x][w]) : m & red[2][w];
+        if (threadIdx.x < 2) atomicMin(&words[threadIdx.x], m);
+        else atomicAnd(&words[2], m);
     }
 }
 
@@ -232,7 +238,7 @@ struct OsScratch {
 // totals into exclusive prefixes.
 constexpr int OS_HREP = 4;
 template <typename Item, int FIELD>
-__global__ void __launch_bounds__(512) os_hist_kernel(const Item* __restrict__ in, int64_t n, uint64_t base, int passes,
+__global__ void __launch_bounds__(512) os_hist_kernel(const Item* __restrict__ in, int64_t n, uint64_t base, int low, int passes,
                                                       OsScratch* __restrict__ sc)
 {
     extern __shared__ unsigned os_h[];  // [pass][digit][copy]
@@ -244,7 +250,7 @@ __global__ void __launch_bounds__(512) os_hist_kernel(const Item* __restrict__ i
     int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     unsigned* mine = os_h + (threadIdx.x & (OS_HREP - 1));
     auto count = [&](const Item& t) {
-        uint64_t k = os_key<Item, FIELD>(t) - base;
+        uint64_t k = (os_key<Item, FIELD>(t) - base) >> low;
         for (int p = 0; p < passes; ++p, k >>= 8) atomicAdd(&mine[(p * OS_BINS + (int)(k & 255)) * OS_HREP], 1u);
     };
     constexpr int U = 4;
@@ -337,7 +343,7 @@ __device__ bool os_look_back(const unsigned long long* status, int64_t tile, int
 
 template <typename Item, int FIELD>
 __global__ void __launch_bounds__(OsShape<Item>::THREADS, OsShape<Item>::MINB)
-    os_pass_kernel(const Item* __restrict__ in, Item* __restrict__ out, int64_t n, uint64_t base, int pass,
+    os_pass_kernel(const Item* __restrict__ in, Item* __restrict__ out, int64_t n, uint64_t base, int shift, int pass,
                    OsScratch* __restrict__ sc, unsigned long long* __restrict__ status,
                    unsigned* __restrict__ err, int64_t mute)
 {
@@ -351,7 +357,6 @@ __global__ void __launch_bounds__(OsShape<Item>::THREADS, OsShape<Item>::MINB)
     __shared__ unsigned ticket;
     __shared__ int ok;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    const int shift = 8 * pass;
     const unsigned agg_tag = 2u * (unsigned)pass + 1u;
     if (tid == 0) {
         ticket = atomicAdd(&sc->ticket[pass], 1u);
@@ -480,6 +485,12 @@ __global__ void __launch_bounds__(1024) os_small_kernel(const Item* __restrict__
         key[i] = i < n ? os_key<Item, FIELD>(in[i]) ^ flip : ~0ULL;
         idx[i] = (unsigned short)i;  // padding: the largest key, the largest positions
     }
+    // Keys in order already (equal ones among them) need no network: 4000
+    // equal keys took 58 us with it.
+    __syncthreads();
+    bool disorder = false;
+    for (int i = threadIdx.x; i + 1 < n; i += blockDim.x) disorder |= key[i] > key[i + 1];
+    if (!__syncthreads_or(disorder)) m = 0;
     // Pairs at stride j <= 32 stay inside the warp's own 64-element blocks:
     // those stages need only a warp barrier.
     bool wide = true;
@@ -510,31 +521,35 @@ __global__ void __launch_bounds__(1024) os_small_kernel(const Item* __restrict__
 // trip: the number of launches depends on it.
 struct OsPlan {
     uint64_t base = 0;
+    int low = 0;  // low bits that all keys share
     int passes = 0;
 };
 
-// Launches the range reading of n > 0 elements into counter words 32 + 2
+// Launches the range reading of n > 0 elements into counter words 128 + 4
 // slot; os_plan_read turns the words into a plan after a synchronisation.
 template <typename Item, int FIELD>
 static int os_plan_launch(pyg_ctx* ctx, const Item* in, int64_t n, bool is_signed, int slot)
 {
     const uint64_t flip = is_signed ? 0x8000000000000000ULL : 0ULL;
-    unsigned long long* words = ctx->dcounters + 32 + 2 * slot;
-    PYG_CUDA(cudaMemsetAsync(words, 0xFF, 16, ctx->stream));
+    unsigned long long* words = ctx->dcounters + 128 + 4 * slot;
+    PYG_CUDA(cudaMemsetAsync(words, 0xFF, 24, ctx->stream));
     os_range_kernel<Item, FIELD><<<grid_for(ctx, n, 512, 4, 4), 512, 0, ctx->stream>>>(in, n, flip, words);
     PYG_LAUNCHED(ctx);
-    PYG_CUDA(cudaMemcpyAsync((unsigned long long*)ctx->pinned + 64 + 2 * slot, words, 16, cudaMemcpyDeviceToHost,
+    PYG_CUDA(cudaMemcpyAsync((unsigned long long*)ctx->pinned + 64 + 4 * slot, words, 24, cudaMemcpyDeviceToHost,
                              ctx->stream));
     return PYG_OK;
 }
 
 static OsPlan os_plan_read(pyg_ctx* ctx, bool is_signed, int slot)
 {
-    const unsigned long long* h = (const unsigned long long*)ctx->pinned + 64 + 2 * slot;
+    const unsigned long long* h = (const unsigned long long*)ctx->pinned + 64 + 4 * slot;
     const uint64_t lo = h[0], hi = ~h[1];
     OsPlan plan;
     plan.base = lo ^ (is_signed ? 0x8000000000000000ULL : 0ULL);
-    plan.passes = hi == lo ? 0 : (64 - __builtin_clzll(hi - lo) + 7) / 8;
+    if (hi != lo) {
+        plan.low = __builtin_ctzll(~h[2]);
+        plan.passes = (64 - __builtin_clzll((hi - lo) >> plan.low) + 7) / 8;
+    }
     return plan;
 }
 
@@ -564,7 +579,7 @@ static int os_passes(pyg_ctx* ctx, const Item* in, Item* dst0, Item* dst1, int64
         PYG_CUDA(cudaMemsetAsync(sc, 0, bytes, ctx->stream));
         const size_t hsm = (size_t)plan.passes * OS_BINS * OS_HREP * 4;
         os_hist_kernel<Item, FIELD>
-            <<<grid_for(ctx, n, 512, 16, 4), 512, hsm, ctx->stream>>>(in, n, plan.base, plan.passes, sc);
+            <<<grid_for(ctx, n, 512, 16, 4), 512, hsm, ctx->stream>>>(in, n, plan.base, plan.low, plan.passes, sc);
         PYG_LAUNCHED(ctx);
         auto kern = os_pass_kernel<Item, FIELD>;
         PYG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM));
@@ -573,7 +588,8 @@ static int os_passes(pyg_ctx* ctx, const Item* in, Item* dst0, Item* dst1, int64
         if (mute == 0) ctx->stall_sort = 0;
         for (int p = 0; p < plan.passes; ++p, mute = -1) {
             Item* dst = p & 1 ? dst1 : dst0;
-            kern<<<(unsigned)tiles, S::THREADS, S::SMEM, ctx->stream>>>(src, dst, n, plan.base, p, sc, status,
+            kern<<<(unsigned)tiles, S::THREADS, S::SMEM, ctx->stream>>>(src, dst, n, plan.base, plan.low + 8 * p, p, sc,
+                                                                        status,
                                                                         (unsigned*)(ctx->dcounters + SORT_ERR_WORD),
                                                                         mute);
             PYG_LAUNCHED(ctx);
