@@ -85,7 +85,10 @@ struct GbrTail {
     bool full = false;
 };
 
-// Adds (sum, cnt) for key k to the HBM table.
+// Adds (sum, cnt) for key k to the HBM table.  Once the table is full the
+// result is discarded and the host redoes the call with a larger one, so
+// nothing more is looked up: without this, 2^25 tuples of 2^23 random keys
+// (no estimate given) spent 245 ms walking full tables.
 __device__ __forceinline__ void gbr_global_add(const GbrArgs& a, uint64_t k, uint64_t sum, uint64_t cnt, GbrTail& z)
 {
     if (k == kEmptyKey) {
@@ -93,8 +96,11 @@ __device__ __forceinline__ void gbr_global_add(const GbrArgs& a, uint64_t k, uin
         z.sent_cnt += cnt;
         return;
     }
+    if (z.full) return;
+    volatile unsigned long long* full = a.flags;
     uint64_t s = reduce_range(mix64(k), a.cap);
     for (uint64_t steps = 0; steps < GBR_PROBE_LIMIT && steps < a.cap; ++steps) {
+        if ((steps & 63) == 63 && *full) break;
         unsigned long long* slot = (unsigned long long*)&a.table[s];
         unsigned long long prev = slot[0];
         if (prev == kEmptyKey) {
@@ -109,6 +115,7 @@ __device__ __forceinline__ void gbr_global_add(const GbrArgs& a, uint64_t k, uin
         s = (s + 1 == a.cap) ? 0 : s + 1;
     }
     z.full = true;
+    *full = 1;
 }
 
 // How the kernels read a tuple: 16-byte (key, value); the same with the two
@@ -340,7 +347,8 @@ __global__ void __launch_bounds__(GBR_PT_THREADS, 2) gbr_part_kernel(GbrArgs a)
     __shared__ long long item;
     GbrTail z;
     for (;;) {
-        if (threadIdx.x == 0) item = (long long)atomicAdd(a.next, 1u);
+        if (threadIdx.x == 0)
+            item = *(volatile unsigned long long*)a.flags ? a.nitems : (long long)atomicAdd(a.next, 1u);
         t.clear(threadIdx.x, GBR_PT_THREADS);
         __syncthreads();
         const long long it = item;
