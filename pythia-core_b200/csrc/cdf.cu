@@ -481,12 +481,12 @@ static int cdf_assign(pyg_ctx* ctx, CdfWork& w, const int64_t* keys, int64_t n, 
     return PYG_OK;  // `init` was staged by the (pageable) copy before it returned
 }
 
-// Packed key words of every step-th tuple (m of them).
-__global__ void key_sample_kernel(const uint8_t* __restrict__ base, int64_t m, int64_t step, int32_t tb, KeySpec ks,
-                                  int64_t* __restrict__ out)
+// Packed key words of one tuple in every `step` (m of n).
+__global__ void key_sample_kernel(const uint8_t* __restrict__ base, int64_t n, int64_t m, int64_t step, int32_t tb,
+                                  KeySpec ks, int64_t* __restrict__ out)
 {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x)
-        out[i] = (int64_t)load_key(base + i * step * tb, ks);
+        out[i] = (int64_t)load_key(base + rj_sample_row(i, step, 1, n) * tb, ks);
 }
 
 }  // namespace pyg
@@ -503,7 +503,7 @@ int estimate_distinct_keys(pyg_ctx* ctx, const uint8_t* base, int64_t n, int32_t
     int64_t* sample = nullptr;
     int rc = dalloc(ctx, (void**)&sample, (size_t)m * 8);
     if (rc) return rc;
-    key_sample_kernel<<<grid_for(ctx, m, 256, 4, 4), 256, 0, ctx->stream>>>(base, m, step, tb, ks, sample);
+    key_sample_kernel<<<grid_for(ctx, m, 256, 4, 4), 256, 0, ctx->stream>>>(base, n, m, step, tb, ks, sample);
     PYG_LAUNCHED(ctx);
     pyg_cdf_train_opts o;
     o.leaves = 64;

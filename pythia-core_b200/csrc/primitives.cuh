@@ -50,7 +50,7 @@ __host__ __device__ __forceinline__ uint64_t packed_to_sortable(uint64_t k, int 
 }
 
 // Distinct-key estimate for n tuples (device, tb bytes each) from the
-// packed keys of a strided sample of CDF_ESTIMATE_SAMPLE tuples: the GEE
+// packed keys of a sample of CDF_ESTIMATE_SAMPLE tuples: the GEE
 // estimate carried by the learned CDF model trained on that sample
 // (cdf.cu).  Sizes hash tables when a caller gives no group estimate.
 constexpr int64_t CDF_ESTIMATE_SAMPLE = (int64_t)1 << 18;

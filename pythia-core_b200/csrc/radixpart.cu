@@ -22,25 +22,6 @@ __device__ __forceinline__ unsigned rj_bin(uint64_t h, int shift, unsigned mask)
     return shift >= 64 ? 0u : (unsigned)(h >> shift) & mask;
 }
 
-// Row that sample i of a layout's histogram reads: one row of every `step`,
-// at a multiple of `spread` that the MurmurHash3 32-bit finaliser of i picks.
-// Rows at a fixed stride see a few values of keys that repeat with the row
-// number (row % 2^16 at a stride of 2^8: one in 2^8), most regions overflow,
-// and the relation is partitioned twice.  spread is 1 for one pass.  For two
-// it is 2: the test of that redo hides keys from the sample in the odd rows
-// of an even stride.
-__device__ __forceinline__ int64_t rj_sample_row(int64_t i, int64_t step, int spread, int64_t n)
-{
-    if (step == 1) return i;
-    unsigned h = (unsigned)i;
-    h ^= h >> 16;
-    h *= 0x85ebca6bu;
-    h ^= h >> 13;
-    h *= 0xc2b2ae35u;
-    h ^= h >> 16;
-    return min(i * step + spread * (int64_t)(((uint64_t)h * (uint64_t)(step / spread)) >> 32), n - 1);
-}
-
 // ---------------------------------------------------------------------------
 // 1. Histogram of the top `bits` hash bits (bits <= 15: 128 KB of shared
 // counters per CTA).

@@ -331,6 +331,25 @@ __host__ __device__ __forceinline__ uint64_t rj_hash(uint64_t k)
     return k * kRjHashMul;
 }
 
+// Row that sample i of a relation reads: one row of every `step`, at a
+// multiple of `spread` that the MurmurHash3 32-bit finaliser of i picks.
+// Rows at a fixed stride see a few values of keys that repeat with the row
+// number (row % 2^16 at a stride of 2^8: one in 2^8): most regions of a layout
+// overflow then, and the relation is partitioned twice.  spread is 1 for one
+// pass.  For two it is 2: the test of that redo hides keys from the sample in
+// the odd rows of an even stride.
+__device__ __forceinline__ int64_t rj_sample_row(int64_t i, int64_t step, int spread, int64_t n)
+{
+    if (step == 1) return i;
+    unsigned h = (unsigned)i;
+    h ^= h >> 16;
+    h *= 0x85ebca6bu;
+    h ^= h >> 13;
+    h *= 0xc2b2ae35u;
+    h ^= h >> 16;
+    return min(i * step + spread * (int64_t)(((uint64_t)h * (uint64_t)(step / spread)) >> 32), n - 1);
+}
+
 // Slot of key k in a shared-memory table of TS slots, for keys of one
 // partition of 2^fb (fb = 0: one partition): multiply-high of the 32 hash
 // bits below the partition bits.

@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 N = 1 << 25
 
 
-@pytest.mark.parametrize("ids,groups", [("uniform", 1 << 23)])
+@pytest.mark.parametrize("ids,groups", [("uniform", 1 << 23), ("periodic", 1 << 16), ("periodic", 1 << 20)])
 def test_cost_of_a_missing_estimate(ctx, torch_cuda, ids, groups):
     torch = torch_cuda
     gen = torch.Generator(device="cuda").manual_seed(groups)
