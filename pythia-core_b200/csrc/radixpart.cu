@@ -194,7 +194,7 @@ struct RJFmt {
     using Out = typename std::conditional<OUT8, unsigned long long, longlong2>::type;
     using Bin = typename std::conditional<IN8, unsigned char, unsigned short>::type;
     static constexpr int TILE =
-        IN8 ? (MODE == RJ_MODE_HASH ? RJ_TILE_8 : RJ_TILE_8M) : (!OUT8 ? RJ_TILE_U : (MODE == RJ_MODE_HASH ? RJ_TILE_P : RJ_TILE_PM));  // the largest
+        IN8 ? (MODE == RJ_MODE_HASH ? RJ_TILE_8 : RJ_TILE_8M) : (!OUT8 ? (MODE == RJ_MODE_HASH ? RJ_TILE_U : RJ_TILE_UM) : (MODE == RJ_MODE_HASH ? RJ_TILE_P : RJ_TILE_PM));  // the largest
 };
 
 __device__ __forceinline__ long long rj_key(const longlong2& t, unsigned long long) { return t.x; }
@@ -249,18 +249,25 @@ __device__ RJTileRange rj_tile_range(const RJPass& a, RJSegCursor& c, long long 
 //     (7.7 ms; 5.1 ms with them taken out).  2 x 512 threads, 4096: 7.1 ms.
 //   packed in and out, hash          probe pass 2 4.03 ms.  256 bins: two
 //     control warps reserve four each per lane (one warp: 4.70 ms).
+//   16-byte in and out, hash         two control warps and 2688-tuple tiles.
+//     With one and 2400, the reservations of 2^9 bins held the tiles up: join
+//     of 2.2 M x 30 M wide keys in one pass 877 -> 719 us, x 100 M 2088 -> 1636,
+//     group-by of 100 M wide keys, G 2^20, 2729 -> 2310; 2^7 bins gain 4% to 6%.
+//     1 x 992 and 5952: 846 us, 1 x 960, two control warps and 5760: 735.
 //   model and range bins wait on their leaf and splitter loads and take
 //     whichever shape measured best: 2.87 and 2.20 ms (model), 3.71 and
-//     2.38 ms (range), group-by 0.72 ms (hash, unpacked).
+//     2.38 ms (range).
 // Against one kernel shape of 2 x 256 or 512 threads without control warps,
 // three barriers per tile and reservations waited for inside a tile: 6.78,
-// 4.66, 3.09, 1.95, 3.92, 3.05 and 0.81 ms.
+// 4.66 (hash), 3.09, 1.95 (model), 3.92 and 3.05 ms (range).
 template <int WORKERS, int CONTROL, int CTAS, int STAGES>
 struct RJShapeOf {
     static constexpr int T = WORKERS, NC = CONTROL, MINB = CTAS, ST = STAGES, THREADS = T + 32 * NC;
 };
 template <bool IN8, bool OUT8, int MODE>
-struct RJShape : RJShapeOf<480, 1, 2, 1> {};  // packed model and range passes; 16-byte tuples in and out
+struct RJShape : RJShapeOf<480, 1, 2, 1> {};  // second and unpacked passes of model and range bins
+template <>
+struct RJShape<false, false, RJ_MODE_HASH> : RJShapeOf<448, 2, 2, 1> {};
 template <>
 struct RJShape<true, true, RJ_MODE_HASH> : RJShapeOf<448, 2, 2, 1> {};
 template <>
@@ -720,8 +727,8 @@ int launch_pass(pyg_ctx* ctx, const RJPass& p, long long ntiles, bool in8, bool 
 
 static void layout_tiles(RJLayout& L, int64_t n, bool pack, bool model)
 {
-    L.tile1 = rj_tile(!pack ? RJ_TILE_U : (model ? RJ_TILE_PM : RJ_TILE_P), n);
-    L.tile2 = rj_tile(!pack ? RJ_TILE_U : (model ? RJ_TILE_8M : RJ_TILE_8), n);
+    L.tile1 = rj_tile(!pack ? (model ? RJ_TILE_UM : RJ_TILE_U) : (model ? RJ_TILE_PM : RJ_TILE_P), n);
+    L.tile2 = rj_tile(!pack ? (model ? RJ_TILE_UM : RJ_TILE_U) : (model ? RJ_TILE_8M : RJ_TILE_8), n);
 }
 
 void layout_exact(const std::vector<unsigned long long>& h, int64_t n, int C, int sub, RJLayout& L, bool pack,

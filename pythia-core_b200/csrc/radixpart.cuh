@@ -37,7 +37,8 @@ namespace pyg {
 
 // Largest tiles (elements) of a partition pass by what it reads and writes
 // (the kernels' shapes are in radixpart.cu).
-constexpr int RJ_TILE_U = 2400;    // 16-byte tuples in and out
+constexpr int RJ_TILE_U = 2688;    // 16-byte tuples in and out: hash bins
+constexpr int RJ_TILE_UM = 2400;   //   model and range bins
 constexpr int RJ_TILE_P = 7936;    // 16-byte tuples in, packed words out: hash bins
 constexpr int RJ_TILE_PM = 3968;   //   model and range bins
 constexpr int RJ_TILE_8 = 5376;    // packed words in and out: hash bins
@@ -237,7 +238,7 @@ int run_passes(pyg_ctx* ctx, const longlong2* in, int64_t n, const RJLayout& L, 
 // reads them), and a last tile's copy of packed words, rounded up to 16
 // bytes, stays inside the buffer.
 constexpr int RJ_DUMP = 8192;
-static_assert(RJ_DUMP >= RJ_TILE_U && RJ_DUMP >= RJ_TILE_P && RJ_DUMP >= RJ_TILE_PM && RJ_DUMP >= RJ_TILE_8 &&
+static_assert(RJ_DUMP >= RJ_TILE_U && RJ_DUMP >= RJ_TILE_UM && RJ_DUMP >= RJ_TILE_P && RJ_DUMP >= RJ_TILE_PM && RJ_DUMP >= RJ_TILE_8 &&
                   RJ_DUMP >= RJ_TILE_8M,
               "a run is at most a tile");
 // Device bytes of a layout's pass buffer of `words` elements.
