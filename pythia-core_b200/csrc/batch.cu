@@ -63,6 +63,8 @@ constexpr int64_t kLargeBuild = (int64_t)1 << 21;
 // bytes each) are queued, the smallest build sides first; the others run as
 // their own joins, whose table is one buffer that they share.
 constexpr uint64_t kQueueSlots = (uint64_t)1 << 26;
+// The smallest work items of untuned plans, in tuples.
+constexpr int64_t kMinGrain = 512;
 // The threshold when even that much memory cannot be had.
 constexpr int64_t kLargeBuildLowMem = (int64_t)1 << 16;
 // Table slots of one wave of queued fragments (16 MB; two waves are live at
@@ -391,12 +393,14 @@ int pyg_batch_create(pyg_ctx* ctx, const pyg_fragment* frags, int32_t n, const p
     }
     *out = nullptr;
     pyg_tuning t = default_tuning();
+    bool untuned = false;
     if (tuning) {
         t = *tuning;
     } else {
         std::lock_guard<std::mutex> g(g_tune_mu);
         auto it = g_tune_cache.find(signature(frags, n));
-        if (it != g_tune_cache.end()) t = it->second;
+        untuned = it == g_tune_cache.end();
+        if (!untuned) t = it->second;
     }
     if (t.block_threads < 64 || t.block_threads > 1024 || (t.block_threads & 31) || t.blocks_per_sm < 1 ||
         t.blocks_per_sm > 16 || !(t.load_factor > 0 && t.load_factor <= 0.9f) || t.chunk_tuples < 256 ||
@@ -470,7 +474,20 @@ int pyg_batch_create(pyg_ctx* ctx, const pyg_fragment* frags, int32_t n, const p
         toff[i] = off;
         off += fd[i].cap;
     }
-    const int64_t grain = t.chunk_tuples;
+    // Work-item grain.  Untuned plans take smaller items where there is little
+    // work: half the size below eight items per resident CTA, then down to
+    // kMinGrain until there is an item for each CTA.  Random 31-bit keys, items
+    // of 4096 and of this size: 44 K tuples 147 and 46 us, 0.5 M 171 and 59,
+    // 7 M 245 and 193 (keys 1..n: 47 and 34, 60 and 47, 99 and 97).
+    int64_t grain = t.chunk_tuples;
+    if (untuned) {
+        int64_t tuples = 0;
+        for (int i = 0; i < n; ++i)
+            if (!is_large[i]) tuples += frags[i].nbuild + frags[i].nprobe;
+        const int64_t ctas = (int64_t)ctx->sm_count * t.blocks_per_sm;
+        if (tuples < 8 * ctas * grain) grain /= 2;
+        while (grain > kMinGrain && tuples < ctas * grain) grain /= 2;
+    }
     for (int i : order) {
         FragDesc& f = fd[i];
         f.build = (const longlong2*)frags[i].build;
