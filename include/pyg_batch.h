@@ -51,9 +51,11 @@ typedef struct pyg_tuning {
     float load_factor;           /* per-fragment table load factor           */
     int32_t chunk_tuples;        /* work-item grain in tuples                */
     int32_t large_build;         /* build tuples from which a fragment runs
-                                    as its own join.  0: 2^21, and those
-                                    beyond 1.3 GB of queued tables (2^16
-                                    when that memory cannot be had)       */
+                                    as its own join.  0: 2^21 (2^20 with
+                                    probes of a quarter of the build or
+                                    more), and those beyond 1.3 GB of
+                                    queued tables (2^16 when that memory
+                                    cannot be had)                        */
 } pyg_tuning;
 
 /* Plans n fragments (tuning NULL: the autotuner's cached choice, else

@@ -63,6 +63,13 @@ constexpr int64_t kLargeBuild = (int64_t)1 << 21;
 // bytes each) are queued, the smallest build sides first; the others run as
 // their own joins, whose table is one buffer that they share.
 constexpr uint64_t kQueueSlots = (uint64_t)1 << 26;
+// Builds from here to kLargeBuild run as their own joins when they have probes
+// to speak of (a quarter of the build or more): two waves of tables of 32 to
+// 64 MB each do not stay in L2, one does.  10 fragments of 2^20..2^21, 41 and
+// 180 M tuples, random 31-bit keys: 1588 and 3212 us queued, 1271 and 2498 on
+// their own; keys 1..n: 651 and 1493, 752 and 1385.  At 2^19..2^20 keys 1..n
+// lose more (494 to 762 us) than random ones gain (1487 to 1335).
+constexpr int64_t kOwnBuild = (int64_t)1 << 20;
 // The smallest work items of untuned plans, in tuples.
 constexpr int64_t kMinGrain = 512;
 // The threshold when even that much memory cannot be had.
@@ -439,7 +446,9 @@ int pyg_batch_create(pyg_ctx* ctx, const pyg_fragment* frags, int32_t n, const p
         uint64_t total_slots = 0;
         for (int i : by_build) {
             const uint64_t cap = (uint64_t)((double)frags[i].nbuild / t.load_factor) + 64;
-            is_large[i] = frags[i].nbuild >= threshold || (automatic && total_slots + cap > kQueueSlots);
+            is_large[i] = frags[i].nbuild >= threshold ||
+                          (automatic && (total_slots + cap > kQueueSlots ||
+                                         (frags[i].nbuild >= kOwnBuild && frags[i].nprobe >= frags[i].nbuild / 4)));
             fd[i].cap = is_large[i] ? 0 : cap;
             total_slots += fd[i].cap;
         }

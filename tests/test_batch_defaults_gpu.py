@@ -52,3 +52,11 @@ def test_little_work_is_spread_over_the_chip(ctx, torch_cuda, sizes):
     pairs, want = fragments(torch_cuda, sizes, 3)
     default = best_run(ctx, torch_cuda, pairs, want)
     assert default < 1.1 * best_run(ctx, torch_cuda, pairs, want, pyg.pyg_tuning(512, 2, 0.5, 4096, 0))
+
+
+def test_large_fragments_with_probes_run_on_their_own(ctx, torch_cuda):
+    """Random keys: 1.26 to 1.42 times the time when queued."""
+    sizes = [((1 << 20) + 100_000 * i, ((1 << 20) + 100_000 * i) * (1 + i % 3)) for i in range(10)]
+    pairs, want = fragments(torch_cuda, sizes, 4)
+    default = best_run(ctx, torch_cuda, pairs, want)
+    assert default < 1.1 * best_run(ctx, torch_cuda, pairs, want, pyg.pyg_tuning(256, 4, 0.5, 4096, 1 << 20))
