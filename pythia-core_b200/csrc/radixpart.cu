@@ -183,7 +183,9 @@ struct RJPass {
 
 // How a pass computes a tuple's bin, fixed per kernel instance so that no
 // per-tuple branch chooses it.
-enum RJMode { RJ_MODE_HASH = 0, RJ_MODE_MODEL = 1, RJ_MODE_RANGE = 2 };
+// HASH9: hash bins, more than 2^8 of them, of a pass from 16-byte tuples to
+// packed words; it has a shape of its own.
+enum RJMode { RJ_MODE_HASH = 0, RJ_MODE_MODEL = 1, RJ_MODE_RANGE = 2, RJ_MODE_HASH9 = 3 };
 
 // Element formats: a pass reads 16-byte tuples (the relation, or unpacked
 // intermediates) or packed 8-byte words, and writes either.  Packed input
@@ -194,7 +196,9 @@ struct RJFmt {
     using Out = typename std::conditional<OUT8, unsigned long long, longlong2>::type;
     using Bin = typename std::conditional<IN8, unsigned char, unsigned short>::type;
     static constexpr int TILE =
-        IN8 ? (MODE == RJ_MODE_HASH ? RJ_TILE_8 : RJ_TILE_8M) : (!OUT8 ? (MODE == RJ_MODE_HASH ? RJ_TILE_U : RJ_TILE_UM) : (MODE == RJ_MODE_HASH ? RJ_TILE_P : RJ_TILE_PM));  // the largest
+        IN8 ? (MODE == RJ_MODE_HASH ? RJ_TILE_8 : RJ_TILE_8M)
+            : !OUT8 ? (MODE == RJ_MODE_HASH ? RJ_TILE_U : RJ_TILE_UM)
+                    : (MODE == RJ_MODE_HASH ? RJ_TILE_P : MODE == RJ_MODE_HASH9 ? RJ_TILE_P9 : RJ_TILE_PM);  // the largest
 };
 
 __device__ __forceinline__ long long rj_key(const longlong2& t, unsigned long long) { return t.x; }
@@ -247,6 +251,10 @@ __device__ RJTileRange rj_tile_range(const RJPass& a, RJSegCursor& c, long long 
 //     the largest tile: a tile reserves one run per bin, and at 2048-tuple
 //     tiles the 64-bit atomics on 128 cursors alone took a third of the pass
 //     (7.7 ms; 5.1 ms with them taken out).  2 x 512 threads, 4096: 7.1 ms.
+//     2^9 bins keep one control warp busy for longer than a tile: two of them
+//     and 960 workers take the join of 2.2 M x 30 M random 31-bit keys from
+//     684 to 588 us, x 100 M from 1930 to 1655.  With 2^7 bins that shape
+//     costs 1.3% (R 2^27 x S 2^30), so it is taken above 2^8 bins only.
 //   packed in and out, hash          probe pass 2 4.03 ms.  256 bins: two
 //     control warps reserve four each per lane (one warp: 4.70 ms).
 //   16-byte in and out, hash         two control warps and 2688-tuple tiles.
@@ -273,6 +281,8 @@ struct RJShape<true, true, RJ_MODE_HASH> : RJShapeOf<448, 2, 2, 1> {};
 template <>
 struct RJShape<false, true, RJ_MODE_HASH> : RJShapeOf<992, 1, 1, 1> {};
 template <>
+struct RJShape<false, true, RJ_MODE_HASH9> : RJShapeOf<960, 2, 1, 1> {};
+template <>
 struct RJShape<false, true, RJ_MODE_MODEL> : RJShapeOf<992, 1, 1, 2> {};
 template <>
 struct RJShape<false, true, RJ_MODE_RANGE> : RJShapeOf<992, 1, 1, 2> {};
@@ -284,7 +294,7 @@ template <bool IN8, bool OUT8, int MODE>
 struct RJPartSmem {
     using F = RJFmt<IN8, OUT8, MODE>;
     // Model and range passes have at most 2^8 bins (RJ_SPLIT_MAX).
-    static constexpr int BINS = MODE == RJ_MODE_HASH ? RJ_LMAX : RJ_SPLIT_MAX;
+    static constexpr int BINS = MODE == RJ_MODE_HASH || MODE == RJ_MODE_HASH9 ? RJ_LMAX : RJ_SPLIT_MAX;
     static constexpr int ST = RJShape<IN8, OUT8, MODE>::ST;
     typename F::In in[ST][F::TILE];
     typename F::Out stage[F::TILE];
@@ -414,6 +424,7 @@ __device__ __forceinline__ void rj_issue_tile(const RJPass& a, RJPartSmem<IN8, O
 //   -- barrier 2
 //   group tile k + 1 in the stage             (reserve the runs of tile k + 1)
 static_assert(sizeof(RJPartSmem<false, true, RJ_MODE_HASH>) <= 232448, "one CTA per SM");
+static_assert(sizeof(RJPartSmem<false, true, RJ_MODE_HASH9>) <= 232448, "one CTA per SM");
 static_assert(sizeof(RJPartSmem<false, true, RJ_MODE_MODEL>) <= 232448, "one CTA per SM");
 static_assert(2 * (sizeof(RJPartSmem<true, true, RJ_MODE_HASH>) + 1024) <= 233472, "two CTAs per SM");
 static_assert(2 * (sizeof(RJPartSmem<true, true, RJ_MODE_RANGE>) + 1024) <= 233472, "two CTAs per SM");
@@ -716,6 +727,7 @@ int launch_pass(pyg_ctx* ctx, const RJPass& p, long long ntiles, bool in8, bool 
     if (ntiles <= 0) return PYG_OK;
     if (p.model.leaf) return launch_pass_m<RJ_MODE_MODEL>(ctx, p, ntiles, in8, out8);
     if (p.nsplit) return launch_pass_m<RJ_MODE_RANGE>(ctx, p, ntiles, in8, out8);
+    if (!in8 && out8 && p.lbits > 8) return launch_pass_t<false, true, RJ_MODE_HASH9>(ctx, p, ntiles);
     return launch_pass_m<RJ_MODE_HASH>(ctx, p, ntiles, in8, out8);
 }
 
@@ -725,16 +737,19 @@ int launch_pass(pyg_ctx* ctx, const RJPass& p, long long ntiles, bool in8, bool 
 
 }  // namespace
 
-static void layout_tiles(RJLayout& L, int64_t n, bool pack, bool model)
+// Tiles of the passes; C: the first pass's bins (launch_pass takes HASH9 above
+// 2^8 of them).
+static void layout_tiles(RJLayout& L, int64_t n, int C, bool pack, bool model)
 {
-    L.tile1 = rj_tile(!pack ? (model ? RJ_TILE_UM : RJ_TILE_U) : (model ? RJ_TILE_PM : RJ_TILE_P), n);
+    const int packing = model ? RJ_TILE_PM : (C > 1 << 8 ? RJ_TILE_P9 : RJ_TILE_P);
+    L.tile1 = rj_tile(!pack ? (model ? RJ_TILE_UM : RJ_TILE_U) : packing, n);
     L.tile2 = rj_tile(!pack ? (model ? RJ_TILE_UM : RJ_TILE_U) : (model ? RJ_TILE_8M : RJ_TILE_8), n);
 }
 
 void layout_exact(const std::vector<unsigned long long>& h, int64_t n, int C, int sub, RJLayout& L, bool pack,
                   bool model)
 {
-    layout_tiles(L, n, pack, model);
+    layout_tiles(L, n, C, pack, model);
     const size_t F = h.size();
     L.sampled = false;
     L.packed = pack;
@@ -776,7 +791,7 @@ static inline unsigned long long sampled_cap(unsigned long long c, long long ste
 void layout_sampled(const std::vector<unsigned long long>& sc, long long step, int64_t n, int C, int sub, RJLayout& L,
                     bool pack, bool model)
 {
-    layout_tiles(L, n, pack, model);
+    layout_tiles(L, n, C, pack, model);
     const size_t F = sc.size();
     L.sampled = true;
     L.packed = pack;

@@ -40,6 +40,7 @@ namespace pyg {
 constexpr int RJ_TILE_U = 2688;    // 16-byte tuples in and out: hash bins
 constexpr int RJ_TILE_UM = 2400;   //   model and range bins
 constexpr int RJ_TILE_P = 7936;    // 16-byte tuples in, packed words out: hash bins
+constexpr int RJ_TILE_P9 = 7680;   //   hash bins, more than 2^8
 constexpr int RJ_TILE_PM = 3968;   //   model and range bins
 constexpr int RJ_TILE_8 = 5376;    // packed words in and out: hash bins
 constexpr int RJ_TILE_8M = 4800;   //   model and range bins
@@ -238,8 +239,8 @@ int run_passes(pyg_ctx* ctx, const longlong2* in, int64_t n, const RJLayout& L, 
 // reads them), and a last tile's copy of packed words, rounded up to 16
 // bytes, stays inside the buffer.
 constexpr int RJ_DUMP = 8192;
-static_assert(RJ_DUMP >= RJ_TILE_U && RJ_DUMP >= RJ_TILE_UM && RJ_DUMP >= RJ_TILE_P && RJ_DUMP >= RJ_TILE_PM && RJ_DUMP >= RJ_TILE_8 &&
-                  RJ_DUMP >= RJ_TILE_8M,
+static_assert(RJ_DUMP >= RJ_TILE_U && RJ_DUMP >= RJ_TILE_UM && RJ_DUMP >= RJ_TILE_P && RJ_DUMP >= RJ_TILE_P9 &&
+                  RJ_DUMP >= RJ_TILE_PM && RJ_DUMP >= RJ_TILE_8 && RJ_DUMP >= RJ_TILE_8M,
               "a run is at most a tile");
 // Device bytes of a layout's pass buffer of `words` elements.
 inline size_t pass_bytes(const RJLayout& L, unsigned long long words)
